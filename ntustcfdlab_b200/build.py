@@ -12,6 +12,8 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -41,19 +43,26 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= _newest_input():
         return OUT
     os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared",
-           "-Xcompiler", "-fPIC,-ffp-contract=off", "-ccbin", "g++",
-           "-cudart", "static", "-o", OUT + ".tmp", *[os.path.join(CSRC, s) for s in SOURCES]]
-    if extra:
-        cmd[1:1] = extra
-    if verbose:
-        print(" ".join(cmd))
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        sys.stderr.write(r.stdout + r.stderr)
+    flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off", "-ccbin", "g++",
+             *(extra or [])]
+
+    def run(cmd):
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        return r.returncode, (" ".join(cmd) + "\n" if verbose else "") + r.stdout + r.stderr
+
+    # the sources compile side by side, then one link
+    with tempfile.TemporaryDirectory(dir=LIB_DIR) as tmp:
+        objs = [os.path.join(tmp, s + ".o") for s in SOURCES]
+        cmds = [[nvcc(), *flags, "-c", "-o", o, os.path.join(CSRC, s)] for s, o in zip(SOURCES, objs)]
+        with ThreadPoolExecutor(len(cmds)) as pool:
+            done = list(pool.map(run, cmds))
+        if all(rc == 0 for rc, _ in done):
+            done.append(run([nvcc(), *ARCH, "-shared", "-ccbin", "g++", "-cudart", "static", "-o", OUT + ".tmp", *objs]))
+    if any(rc for rc, _ in done):
+        sys.stderr.write("".join(text for _, text in done))
         raise RuntimeError("nvcc failed")
-    if verbose and (r.stdout or r.stderr):
-        print(r.stdout + r.stderr)
+    if verbose:
+        print("".join(text for _, text in done))
     os.replace(OUT + ".tmp", OUT)
     return OUT
 

@@ -8,9 +8,8 @@
 namespace ntcfd {
 
 struct GridBar {
-    // low 32 bits: arrivals since the launch began; high 32 bits: the sum over the
-    // sweeps' closing barriers of the CTAs whose max |change| was above zeta, plus
-    // 2^20 per CTA whose max was not finite (k_defect zeroes the word)
+    // low 32 bits: arrivals since the launch began; high 32 bits: the sum of the flags
+    // added with them (k_defect zeroes the word)
     unsigned long long word;
     int err;
     int pad;

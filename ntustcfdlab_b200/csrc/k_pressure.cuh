@@ -17,97 +17,11 @@
 
 #include <type_traits>
 
+#include "k_exchange.cuh"
+#include "k_sor_math.cuh"
 #include "ntcfd_common.cuh"
 
 namespace ntcfd {
-
-template <class Tc>
-struct SorCoef {
-    const Tc *cE, *cW, *cN, *cS, *cF, *cB;
-};
-
-__device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
-
-// 1 / sum of the six coefficients (correctly rounded reciprocal)
-template <class Tc>
-__device__ __forceinline__ Tc rdiag_of(const SorCoef<Tc>& s, int i, int j, int k) {
-    return rcp_rn(((s.cE[i] + s.cW[i]) + (s.cN[j] + s.cS[j])) + (s.cF[k] + s.cB[k]));
-}
-
-// Explicitly rounded operations: every kernel that evaluates a sweep or a
-// defect uses these, so the resident and streaming paths round alike
-// whatever the compiler would contract.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-
-// One SOR update of a cell of the correction e (GS.f90:43-53 in the form
-// eNew = rdiag * sum_nb c_nb e_nb + d): returns eNew - e0 and the relaxed
-// value e0 + omega (eNew - e0) in *e1.
-template <class Tc>
-__device__ __forceinline__ Tc sor_update(Tc cE, Tc oE, Tc cW, Tc oW, Tc cN, Tc oN, Tc cS, Tc oS, Tc cF,
-                                         Tc oF, Tc cB, Tc oB, Tc rd, Tc d, Tc e0, Tc om, Tc* e1) {
-    Tc s = mul_rn(cE, oE);
-    s = fma_rn(cW, oW, s);
-    s = fma_rn(cN, oN, s);
-    s = fma_rn(cS, oS, s);
-    s = fma_rn(cF, oF, s);
-    s = fma_rn(cB, oB, s);
-    const Tc diff = sub_rn(fma_rn(rd, s, d), e0);
-    *e1 = fma_rn(om, diff, e0);
-    return diff;
-}
-
-// FP64 defect of a cell, d = rdiag * sum_nb c_nb p_nb - b' - p (the reference
-// sweep's fixed-point residual), rd = rdiag_of of the cell: the same sums as
-// sor_update.
-__device__ __forceinline__ double defect_value(double cE, double pe, double cW, double pw, double cN, double pn,
-                                               double cS, double ps, double cF, double pf, double cB, double pb,
-                                               double rd, double bv, double pc) {
-    double s = mul_rn(cE, pe);
-    s = fma_rn(cW, pw, s);
-    s = fma_rn(cN, pn, s);
-    s = fma_rn(cS, ps, s);
-    s = fma_rn(cF, pf, s);
-    s = fma_rn(cB, pb, s);
-    return sub_rn(fma_rn(rd, s, -bv), pc);
-}
-
-// FP64 reciprocal of a coefficient sum (positive and finite): the hardware's
-// approximate double reciprocal refined by two Newton-Raphson steps
-// x' = x + x (1 - s x), each of which squares the relative error.
-__device__ __forceinline__ double rdiag64(double s) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(s));
-    double r = fma_rn(-s, x, 1.0);
-    x = fma_rn(x, r, x);
-    r = fma_rn(-s, x, 1.0);
-    x = fma_rn(x, r, x);
-    return x;
-}
-
-// The FP64 defect of p + e from the defect d of p and the correction e of a
-// defect-correction cycle: since the operator is linear,
-//     d' = rdiag sum c (p+e)_nb - b' - (p+e) = d + rdiag sum_nb c_nb e_nb - e,
-// formed in FP64 with the FP64 coefficients from the cycle's (exact) Tc
-// values of e; rdiag is rdiag64 of the FP64 coefficient sum.  Both SOR paths
-// restart a cycle with it.
-template <class Tc>
-__device__ __forceinline__ double defect_update(double cE, Tc eE, double cW, Tc eW, double cN, Tc eN, double cS,
-                                                Tc eS, double cF, Tc eF, double cB, Tc eB, Tc d, Tc e) {
-    double s = mul_rn(cE, (double)eE);
-    s = fma_rn(cW, (double)eW, s);
-    s = fma_rn(cN, (double)eN, s);
-    s = fma_rn(cS, (double)eS, s);
-    s = fma_rn(cF, (double)eF, s);
-    s = fma_rn(cB, (double)eB, s);
-    const double x = rdiag64(((cE + cW) + (cN + cS)) + (cF + cB));
-    return sub_rn(fma_rn(x, s, (double)d), (double)e);
-}
 
 // Column-walking kernel (k_rhs): a 32 x 8 block covers (i, j) and
 // walks the planes of its chunk k0..k1 (chunk = blockIdx.z, chunks of
@@ -158,15 +72,14 @@ __global__ void __launch_bounds__(kWalkBX * kWalkBY) k_rhs(Geom g, SorCoef<doubl
 // on (ctl->cycles > 0), d is instead updated from the last cycle's correction
 // (defect_update) and e is left for k_clear_e.  Inside the step graph
 // (in_graph = 1) it also arms the inner loop's condition.
-// For the resident path (ring != null) it also clears the ring of sweep
-// maxima and the grid barrier the next kernel uses, and with begin = 1 it
-// starts the solve (the counters k_sor_begin resets).
+// For the resident path (rs != null) it also clears the counters the next kernel
+// uses, and with begin = 1 it starts the solve (the counters k_sor_begin resets).
 template <class Tc>
 __global__ void __launch_bounds__(256) k_defect(Geom g, SorCoef<double> sc, const double* p,
                                                 const double* b, Tc* dR, Tc* dB, Tc* eR, Tc* eB,
                                                 const Tc* rdR, const Tc* rdB, Ctl* ctl,
                                                 cudaGraphConditionalHandle inner, int in_graph,
-                                                unsigned long long* ring, unsigned int* bar, int begin, int incr) {
+                                                ResSync* rs, int begin, int incr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -184,8 +97,12 @@ __global__ void __launch_bounds__(256) k_defect(Geom g, SorCoef<double> sc, cons
         }
         ctl->inner = 0;
         if (in_graph) cudaGraphSetConditional(inner, 1u);
-        if (ring) { ring[0] = 0ULL; ring[1] = 0ULL; ring[2] = 0ULL; }
-        if (bar) { bar[0] = 0u; bar[1] = 0u; bar[2] = 0u; }   // GridBar word and err
+        if (rs) {                       // the resident kernel's counters (not its sequence number)
+            rs->bar.word = 0ULL;
+            rs->bar.err = 0;
+            for (int q = 0; q < 4; ++q) rs->cnt[0][q] = rs->cnt[1][q] = 0ULL;
+            rs->last = 0ULL;
+        }
     }
     if (i > g.nx || j > g.ny || k > g.nz) return;
     const long long q = spl(g, (i + 2) >> 1, j, k);

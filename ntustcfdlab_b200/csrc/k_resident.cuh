@@ -2,25 +2,38 @@
 // in one persistent cooperative kernel, with the correction e resident in
 // shared memory.
 //
-// The interior rows (j,k) are split into nbj x nbk bricks of at most JB x KB
-// rows; CTA b owns brick (b % nbj, b / nbj) and keeps e of both colours for
+// The interior rows (j,k) are split into nbj x nbk bricks of balanced sizes;
+// CTA b owns brick (b % nbj, b / nbj) and keeps e of both colours for
 // its rows in shared memory (colour-split rows of mx entries, see
 // ntcfd_common.cuh) with a one-row ring, and the defect d and 1/diag rd of its
 // rows when they fit.  The ring rows of a domain boundary stay 0; the others
-// hold the neighbour bricks' boundary rows, which every CTA publishes to the
-// global e arrays as it updates them and copies into its ring ("fill") once
-// per half-sweep.  A sweep runs
-//     red:   [fill the black ring] -> interior rows -> edge rows -> arrive
-//     black: interior rows (own red values only) -> wait -> fill the red ring
-//            -> edge rows -> max |change| -> grid barrier,
-// so the fill latency overlaps the red interior rows and the first barrier
-// overlaps the black interior rows.  The sweep count, the stop rule
-// (GS.f90:11,53), the count of correction cycles and the final p += e run
-// inside the kernel, and so do the restarts of the defect correction: when a
+// hold the neighbour bricks' boundary rows.  A half-sweep runs
+//     interior rows -> ring -> edge rows (published) -> CTA barrier.
+//
+// The ring (k_exchange.cuh).  The owner of an edge cell stores each new value as
+// one word with a sequence number into the inbox of the CTA that needs it, and that
+// CTA polls the words into its ring: the hand-over costs one trip through L2, which
+// the interior rows cover.  An inbox holds one word per ring cell and colour.  A
+// CTA publishes a colour only after a CTA barrier that follows its reading of the
+// other colour, which its neighbour published after reading the first: no word is
+// overwritten unread.  A grid barrier per half-sweep and a copy of the published
+// rows afterwards, which this replaces, took 3.4 us of an 8.0 us FP32 sweep at 128^3.
+// A sweep takes 6.2 us at 128^3 FP32 (8.0 before), 11.4 FP64 (11.8), 3.3 us at 40^3
+// (5.3) and 3.5 us at 32x96x96 (6.2): on small grids the hand-over, some 1.5 us per
+// half-sweep from a store to its sight by the neighbour, is all that is left; at 128^3
+// the shared-memory pipe takes the larger part (24 words per 64 cells and pass).
+//
+// The stop rule (GS.f90:11,53).  A sweep ends the solve when no cell of either colour
+// changed by more than zeta.  Every CTA adds the verdict of its red half to a
+// counter when that half ends and reads the sum when its black half has ended: one
+// red change above zeta anywhere already decides that the solve goes on, so the
+// black half's verdicts are waited for only in a sweep whose red half had none.
+// The sweep count, the count of correction cycles and the final p += e run inside
+// the kernel, and so do the restarts of the defect correction: when a
 // cycle ends on its length (cycle_len sweeps), the kernel refreshes the black
 // ring, adds e to p and updates d to the FP64 defect of p + e
 // (defect_update: d + rdiag sum c e_nb - e, in FP64, from the exact FP32
-// values of e) without a grid barrier, then sweeps on from e = 0.  The first
+// values of e), then sweeps on from e = 0.  The first
 // defect of the solve comes from k_defect.
 //
 // A lane updates two cells at a time with every load issued before any
@@ -32,14 +45,13 @@
 // shared-memory allocation (or the padded global arrays); a lane past the
 // row's last cell stores nothing and leaves the change maximum alone.
 //
-// The grid barrier spins with a bounded number of polls; a CTA that gives
-// up sets bar->err, and every CTA leaves the sweep loop at the next barrier,
-// so the kernel always ends.  The host reports NTCFD_ETIMEOUT.
+// Every wait is bounded: a CTA that gives up sets sync->bar.err, the others leave
+// the sweep loop at their next wait, and the host reports NTCFD_ETIMEOUT.
 #pragma once
 
 #include <type_traits>
 
-#include "k_gridbar.cuh"
+#include "k_exchange.cuh"
 #include "k_pressure.cuh"
 #include "ntcfd_common.cuh"
 
@@ -50,11 +62,12 @@ enum { kResNarrow = 0, kResWide1 = 1, kResWide = 2 };
 
 struct Brick {
     int nbj, nbk;    // bricks along j and k
-    int JB, KB;      // rows per brick (the last brick may hold fewer)
+    int JB, KB;      // rows of the largest brick
     int mx;          // colour-split row length (compact index m = 0..mx-1)
     int cache_d;     // 1: d of the brick lives in shared memory too
     int cache_rd;    // 1: rd of the brick lives in shared memory too
     int mode;        // kResNarrow, kResWide1 or kResWide (res_mode(nx))
+    int inbox;       // ring words per CTA and colour
 };
 
 // Cells of a colour in a row: (nx + r) / 2 for parity r; at most (nx + 1) / 2.
@@ -70,17 +83,17 @@ inline size_t resident_smem(const Brick& b, int nx) {
     const size_t brick = (size_t)b.JB * b.KB * b.mx;
     const size_t arrays = sizeof(Tc) * (2 * tile + 2 * (size_t)(nx + 4) + 2 * (size_t)(b.JB + b.KB) +
                                         (b.cache_d ? 2 * brick : 0) + (b.cache_rd ? 2 * brick : 0));
-    // + row table (int4 offsets and four coefficients per row), + the face-ring list
-    // (int2 per ring row), + slack: the loads of a lane past a row's last cell may
+    // + row table (int4 offsets, four coefficients and two inbox places per row), + the
+    // ring list (int2 per ring row), + slack: the loads of a lane past a row's last cell may
     // reach up to 64 elements beyond the tiles
     const size_t rows = (size_t)b.JB * b.KB;
-    return ((arrays + 15) & ~size_t(15)) + rows * (16 + 4 * sizeof(Tc)) + 2 * (size_t)(b.JB + b.KB) * 8 +
+    return ((arrays + 15) & ~size_t(15)) + rows * (16 + 4 * sizeof(Tc) + 8) + 2 * (size_t)(b.JB + b.KB) * 8 +
            64 * sizeof(Tc);
 }
 
-// ring values a thread holds in flight while it updates interior rows (32 bytes)
+// ring words a thread holds in flight
 template <class Tc>
-constexpr int kFillOf = 32 / (int)sizeof(Tc);
+constexpr int kFillOf = 24 / (int)sizeof(Tc);
 
 constexpr unsigned int kNanFlag = 1u << 20;   // high-half flag of a CTA whose max |change| was not finite
 
@@ -113,7 +126,7 @@ struct ResRow {
     const Tc* R;      // rd of the row, likewise
     Tc cN, cS, cF, cB;
     int par;          // (j + k) & 1 of the row
-    long long gr;     // global colour-split row start
+    unsigned long long *pubA, *pubB;   // an edge row's words in its neighbours' inboxes (t = 0; null: none)
 };
 
 // The loaded operands of one cell.
@@ -122,16 +135,17 @@ struct ResIn {
     Tc oE, oW, oN, oS, oF, oB, e0, d, rd;
 };
 
-// Loads of the cell at own index m (t + 2 - R) of a row of parity R, all from
-// shared memory: the tile's face ring holds the neighbour bricks' rows of the
-// other colour (fill_ring).  d may be rewritten inside the launch by this CTA
+// Loads of cell t of a row, at own index m = t + 2 - parity, all from shared memory:
+// the tile's ring holds the neighbour bricks' rows of the other colour (fill).
+// The east and west neighbours sit at t + 2 and t + 1 whatever the parity.
+// d may be rewritten inside the launch by this CTA
 // only: a plain (L1-coherent) load when it is global.
-template <class Tc, bool CD, bool CR, int R>
-__device__ __forceinline__ ResIn<Tc> res_load(const ResRow<Tc>& w, int m, int mx, int plane) {
+template <class Tc, bool CD, bool CR>
+__device__ __forceinline__ ResIn<Tc> res_load(const ResRow<Tc>& w, int t, int m, int mx, int plane) {
     ResIn<Tc> x;
     const Tc* o = w.O + m;
-    x.oE = o[R];
-    x.oW = o[R - 1];
+    x.oE = w.O[t + 2];
+    x.oW = w.O[t + 1];
     x.oN = o[mx];
     x.oS = o[-mx];
     x.oF = o[plane];
@@ -142,35 +156,44 @@ __device__ __forceinline__ ResIn<Tc> res_load(const ResRow<Tc>& w, int m, int mx
     return x;
 }
 
-// The update of a loaded cell; stores e (and publishes it for an EDGE row)
-// and takes the change into the maximum only when ok.
+// The update of a loaded cell t of a row; stores e and takes the change into the
+// maximum only when ok.  A cell of an EDGE row goes to the neighbours' inboxes too
+// (ring: a cell of the ring; 0 where a row is a cell shorter than the ring).
 template <class Tc, bool EDGE, class B>
-__device__ __forceinline__ void res_finish(const ResIn<Tc>& x, const ResRow<Tc>& w, int m, Tc cE, Tc cW, Tc om,
-                                           bool ok, Tc* Ec, B& ch) {
+__device__ __forceinline__ void res_finish(const ResIn<Tc>& x, const ResRow<Tc>& w, int t, int m, Tc cE, Tc cW, Tc om,
+                                           bool ok, bool ring, unsigned int seq, B& ch) {
     Tc e1;
     const Tc diff = sor_update(cE, x.oE, cW, x.oW, w.cN, x.oN, w.cS, x.oS, w.cF, x.oF, w.cB, x.oB, x.rd, x.d,
                                x.e0, om, &e1);
     if (ok) {
         w.W[m] = e1;
-        if (EDGE) Ec[w.gr + m] = e1;
         const B db = abs_bits(diff);
         ch = db > ch ? db : ch;
+    }
+    if (EDGE) {
+        using Word = RingWord<Tc>;
+        const Tc v = ok ? e1 : Tc(0);
+        if (ring && w.pubA) Word::store(w.pubA + t * Word::n, v, seq);
+        if (ring && w.pubB) Word::store(w.pubB + t * Word::n, v, seq);
     }
 }
 
 template <class Tc, int NT, bool CD, bool CR, int MODE>
 __global__ void __launch_bounds__(NT, 1)
 k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const double* __restrict__ b,
-               Tc* __restrict__ eRg, Tc* __restrict__ eBg, Tc* __restrict__ dRg, Tc* __restrict__ dBg,
-               const Tc* __restrict__ rdRg, const Tc* __restrict__ rdBg, Ctl* ctl, GridBar* bar,
-               double omega, double zeta, int itmax, int cycle_len, int check_every,
-               unsigned long long* ring) {
+               Tc* __restrict__ dRg, Tc* __restrict__ dBg, const Tc* __restrict__ rdRg,
+               const Tc* __restrict__ rdBg, Ctl* ctl, ResSync* sync, unsigned long long* boxes,
+               double omega, double zeta, int itmax, int cycle_len, int check_every) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using B = decltype(abs_bits(Tc(0)));
     constexpr int kFill = kFillOf<Tc>;
-    __shared__ int s_flag;
-    __shared__ unsigned int s_hi;
-    __shared__ B s_red[NT / 32];
+    using Word = RingWord<Tc>;
+    __shared__ int s_flag, s_fail[2], s_nan[2];   // by the sweep's parity, so that a thread ahead writes the other
+    // verdicts of the sweep (CTAs above zeta, kNanFlag per NaN): red half, black half (of the
+    // sweep before until this one's is waited for)
+    __shared__ uint2 s_vd;
+    __shared__ unsigned int s_prev[2][4];         // high halves of the counters at their last use
+    __shared__ B s_red_max[NT / 32];
     const int JB = br.JB, KB = br.KB, mx = br.mx;
     const int RS = JB + 2;                    // rows per k-plane of the tile
     const int plane = RS * mx;
@@ -194,21 +217,22 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     Tc* const arrays_end = CR ? R1 + brick : (CD ? D1 + brick : D0);
     // row table: per row of the brick, in sweep order (edge rows first), the tile row
     // start, the brick row start of d/rd, the global colour-split row start and
-    // (j+k)&1; and the row's cN, cS, cF, cB.  Then the face ring: per ring row of
-    // the tile that stands for a row of a neighbour brick, its tile row start and
-    // global colour-split row start (y = -1: a domain ghost row, kept at 0).
+    // (j+k)&1; the row's cN, cS, cF, cB; its places in the neighbours' inboxes.  Then the
+    // ring: per row of a neighbour brick (inbox order) its tile row start and (j+k)&1.
     const size_t toff = ((size_t)((unsigned char*)arrays_end - smem_raw) + 15) & ~size_t(15);
     int4* const rowT = reinterpret_cast<int4*>(smem_raw + toff);
     Tc* const rowC = reinterpret_cast<Tc*>(rowT + JB * KB);
-    int2* const ringT = reinterpret_cast<int2*>(rowC + 4 * JB * KB);
+    int2* const pubT = reinterpret_cast<int2*>(rowC + 4 * JB * KB);
+    int2* const ringT = pubT + JB * KB;
     constexpr int NWARP = NT / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tid = threadIdx.x;
 
     const int bj = blockIdx.x % br.nbj, bk = blockIdx.x / br.nbj;
-    const int j0 = 1 + bj * JB, k0 = 1 + bk * KB;
-    const int nj = max(0, min(g.ny, j0 + JB - 1) - j0 + 1);
-    const int nk = max(0, min(g.nz, k0 + KB - 1) - k0 + 1);
+    const int j0 = 1 + brick_start(bj, g.ny, br.nbj), nj = 1 + brick_start(bj + 1, g.ny, br.nbj) - j0;
+    const int k0 = 1 + brick_start(bk, g.nz, br.nbk), nk = 1 + brick_start(bk + 1, g.nz, br.nbk) - k0;
+    const bool jlo = bj > 0, jhi = bj < br.nbj - 1, klo = bk > 0, khi = bk < br.nbk - 1;   // neighbouring bricks
+    const bool multi = gridDim.x > 1;
     const int ys = g.mxp, zs = (int)g.mz;   // colour-split row and plane pitch
     // cells of a colour in a row of parity r
     const int nown0 = g.nx / 2, nown1 = (g.nx + 1) / 2;
@@ -231,22 +255,24 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     const int nrows = nj * nk;
     const int ni = (nj > 2 && nk > 2) ? (nj - 2) * (nk - 2) : 0;   // interior rows
     const int ne = nrows - ni;                                       // edge rows
-    const int nring = 2 * (nj + nk);
+    // the ring rows in the order of the inbox: faces j-low, j-high (nk rows each), k-low,
+    // k-high (nj rows each), those without a neighbour left out
+    const int fj = (jlo ? nk : 0) + (jhi ? nk : 0), nring = fj + (klo ? nj : 0) + (khi ? nj : 0);
     for (int q = tid; q < nring; q += NT) {
-        // faces j-low, j-high (nk rows each), then k-low, k-high (nj rows each)
         int jl, kl;
-        if (q < 2 * nk) {
+        if (q < fj) {
             kl = q % nk + 1;
-            jl = q < nk ? 0 : nj + 1;
+            jl = jlo && q < nk ? 0 : nj + 1;
         } else {
-            const int r = q - 2 * nk;
+            const int r = q - fj;
             jl = r % nj + 1;
-            kl = r < nj ? 0 : nk + 1;
+            kl = klo && r < nj ? 0 : nk + 1;
         }
-        const int j = j0 + jl - 1, k = k0 + kl - 1;
-        const bool inner = j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
-        ringT[q] = make_int2((kl * RS + jl) * mx, inner ? ys * (j + 1) + zs * (k + 1) : -1);
+        ringT[q] = make_int2((kl * RS + jl) * mx, (j0 + jl - 1 + k0 + kl - 1) & 1);
     }
+    // planes of the neighbours along k (those along j have this brick's)
+    const int nkl = klo ? k0 - 1 - brick_start(bk - 1, g.nz, br.nbk) : 0;
+    const int nkh = khi ? brick_start(bk + 2, g.nz, br.nbk) - brick_start(bk + 1, g.nz, br.nbk) : 0;
     for (int er = tid; er < nrows; er += NT) {
         int jl, kl;
         brick_row(er, nj, nk, ni, ne, jl, kl);
@@ -257,7 +283,25 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
         rowC[4 * er + 1] = sc.cS[j];
         rowC[4 * er + 2] = sc.cF[k];
         rowC[4 * er + 3] = sc.cB[k];
+        // the row's ring row in a neighbour: at most one along j and one along k (a brick
+        // that has neighbours on both sides of a direction is two rows thick or more)
+        int pj = -1, pk = -1;
+        if (jl == 1 && jlo)                    // the j-high face of brick bj - 1
+            pj = (int)(blockIdx.x - 1) * 2 * br.inbox + ((bj > 1 ? nk : 0) + kl - 1) * nown1;
+        else if (jl == nj && jhi)              // the j-low face of brick bj + 1
+            pj = (int)(blockIdx.x + 1) * 2 * br.inbox + (kl - 1) * nown1;
+        if (kl == 1 && klo)                    // the k-high face of brick bk - 1
+            pk = (int)(blockIdx.x - br.nbj) * 2 * br.inbox +
+                 ((jlo ? nkl : 0) + (jhi ? nkl : 0) + (bk > 1 ? nj : 0) + jl - 1) * nown1;
+        else if (kl == nk && khi)              // the k-low face of brick bk + 1
+            pk = (int)(blockIdx.x + br.nbj) * 2 * br.inbox + ((jlo ? nkh : 0) + (jhi ? nkh : 0) + jl - 1) * nown1;
+        pubT[er] = pj >= 0 ? make_int2(pj, pk) : make_int2(pk, -1);
     }
+    if (tid == 0) {
+        s_fail[0] = s_fail[1] = s_nan[0] = s_nan[1] = 0;
+        s_vd = make_uint2(0u, 0u);
+    }
+    if (tid < 8) s_prev[tid >> 2][tid & 3] = 0u;
     if (CD || CR) {
         // d (the solve's first defect, from k_defect) and rd of the brick: one warp per
         // row, lanes along m
@@ -278,29 +322,33 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
         }
     }
     __syncthreads();
-    // lane coefficients of the one- and two-row instances: the cells t = lane (and
-    // t = lane + 32) of a row of parity r sit at i = 2t + 2 - r (past the row's end
+    // the lane's cell t in the narrow form, and its row among the rpw side by side
+    const int rpw = MODE == kResNarrow ? 32 / nown1 : 1;
+    const int sub = MODE == kResNarrow ? lane / nown1 : 0, lt = lane - sub * nown1;
+    // lane coefficients of the one- and two-row instances: the cells t = lt (and
+    // t = lt + 32) of a row of parity r sit at i = 2t + 2 - r (past the row's end
     // they read other table entries, never used)
     Tc cEr[2][2], cWr[2][2];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int i = 2 * (lane + 32 * h) + 2 - r;
+            const int i = 2 * (lt + 32 * h) + 2 - r;
             cEr[r][h] = MODE == kResWide ? Tc(0) : cEs[min(i, g.nx + 2)];
             cWr[r][h] = MODE == kResWide ? Tc(0) : cWs[min(i, g.nx + 2)];
         }
 
-    unsigned int nbar = 0;   // grid barriers of this launch passed so far
-    unsigned int hi_prev = 0u;   // high half of the barrier word at the last closing barrier
-    bool tested = false;         // a stop test ran in this launch
     const unsigned int nblocks = gridDim.x;
+    const unsigned int seq0 = sync->seq;
+    const bool ctrl = multi && tid == NT / 2;   // the thread that talks to the counters
     const int ik0 = ctl->ik;
     const Tc om = (Tc)omega;
     int done = 0;        // sweeps of this launch
     int done_c = 0;      // sweeps of the current cycle
     int restarts = 0;
     bool conv = false, nonfinite = false, failed = false;
+    bool tested = false, prev_tested = false;   // a stop test ran; in the sweep before
+    B chs = B(0);        // this thread's max |change| of the last sweep
     double last = 0.0;
 
     // p += e over the brick (natural <- shared memory); one warp per pair of rows,
@@ -427,60 +475,50 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     };
 
 
-    // ---- the face ring of the other colour's tile from the neighbour bricks' rows,
-    // published before the last grid barrier: loads through L2 only (the rows change
-    // between half-sweeps, and this SM's L1 may hold an older copy).  fill_issue puts
-    // the first kFill per thread in flight into registers; fill_commit stores them,
-    // moves any further ones and ends with a CTA barrier.  For the red half the ring
-    // is the black one (c = 0), for the black half the red one.
-    const unsigned int mMX = 0xffffffffu / (unsigned)mx + 1u;   // q / mx, exact for q * mx < 2^32 (mx >= 3)
-    const int ring_tot = nring * mx;
-    auto fill_issue = [&](int c, Tc (&v)[kFill]) {
-        const Tc* const Og = c ? eRg : eBg;
-#pragma unroll
-        for (int u = 0; u < kFill; ++u) {
-            const int q = min(tid + NT * u, ring_tot - 1);
-            const unsigned int r = __umulhi((unsigned)q, mMX);
-            const int2 rr = ringT[r];
-            v[u] = __ldcg(Og + max(rr.y, 0) + (q - (int)r * mx));
-        }
-    };
-    auto fill_commit = [&](int c, const Tc (&v)[kFill]) {
-        Tc* const O = c ? S0 : S1;
-        const Tc* const Og = c ? eRg : eBg;
-#pragma unroll
-        for (int u = 0; u < kFill; ++u) {
-            const int q = tid + NT * u;
-            if (q >= ring_tot) continue;
-            const unsigned int r = __umulhi((unsigned)q, mMX);
-            const int2 rr = ringT[r];
-            if (rr.y >= 0) O[rr.x + (q - (int)r * mx)] = v[u];
-        }
-        for (int q0 = NT * kFill; q0 < ring_tot; q0 += NT * kFill) {
-            Tc w[kFill];
-            int dst[kFill];
-#pragma unroll
-            for (int u = 0; u < kFill; ++u) {
-                const int q = min(q0 + tid + NT * u, ring_tot - 1);
-                const unsigned int r = __umulhi((unsigned)q, mMX);
-                const int m = q - (int)r * mx;
-                const int2 rr = ringT[r];
-                dst[u] = rr.y >= 0 && q0 + tid + NT * u < ring_tot ? rr.x + m : -1;
-                w[u] = __ldcg(Og + max(rr.y, 0) + m);
-            }
+    // ---- the ring of colour oc from this CTA's inbox, words numbered seq: kFill words per
+    // thread in flight, polled until they carry the number.  A CTA barrier follows.
+    const unsigned int mH = 0xffffffffu / (unsigned)nown1 + 1u;   // q / nown1, exact for q * nown1 < 2^32
+    const int ring_tot = nring * nown1;
+    const size_t boxw = (size_t)br.inbox * Word::n;               // 8-byte words of a colour
+    auto fill = [&](int oc, unsigned int seq, int par) {
+        Tc* const O = oc ? S1 : S0;
+        const unsigned long long* const bx = boxes + ((size_t)blockIdx.x * 2 + oc) * boxw;
+        for (int q0 = 0; q0 < ring_tot; q0 += NT * kFill) {
+            Word w[kFill];
 #pragma unroll
             for (int u = 0; u < kFill; ++u)
-                if (dst[u] >= 0) O[dst[u]] = w[u];
+                w[u].load(bx + (size_t)min(q0 + tid + NT * u, ring_tot - 1) * Word::n);
+            for (unsigned int polls = 0;; ++polls) {
+                bool all = true;
+#pragma unroll
+                for (int u = 0; u < kFill; ++u) all = all && w[u].has(seq);
+                if (all) break;
+                if ((polls & 255u) == 255u && ring_lost(sync, polls)) {
+                    s_fail[par] = 1;
+                    break;
+                }
+#pragma unroll
+                for (int u = 0; u < kFill; ++u)
+                    w[u].load(bx + (size_t)min(q0 + tid + NT * u, ring_tot - 1) * Word::n);
+            }
+#pragma unroll
+            for (int u = 0; u < kFill; ++u) {
+                const int q = q0 + tid + NT * u;
+                if (q >= ring_tot) continue;
+                const unsigned int r = __umulhi((unsigned)q, mH);
+                const int2 rr = ringT[r];
+                // cell t of the row sits at m = t + 2 - parity
+                O[rr.x + (q - (int)r * nown1) + 2 - (rr.y ^ oc)] = w[u].value();
+            }
         }
-        __syncthreads();
     };
 
     // ---- one half-sweep of colour c over rows [e0r, e1r) (edge rows: EDGE)
-    auto rows_pass = [&](auto edge_tag, int c, int e0r, int e1r, B& ch) {
+    auto rows_pass = [&](auto edge_tag, int c, int e0r, int e1r, unsigned int seq, B& ch) {
         constexpr bool EDGE = decltype(edge_tag)::value;
         Tc* const W = c ? S1 : S0;
         const Tc* const O = c ? S0 : S1;
-        Tc* const Ec = c ? eBg : eRg;
+        unsigned long long* const Ec = boxes + (size_t)c * boxw;
         const Tc* const Dg = c ? dBg : dRg;
         const Tc* const Rg = c ? rdBg : rdRg;
         const Tc* const Ds = c ? D1 : D0;
@@ -492,150 +530,179 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
             w.W = W + rt.x;
             w.D = CD ? Ds + rt.y : Dg + rt.z;
             w.R = CR ? Rs + rt.y : Rg + rt.z;
-            w.cN = rowC[4 * er];
-            w.cS = rowC[4 * er + 1];
-            w.cF = rowC[4 * er + 2];
-            w.cB = rowC[4 * er + 3];
+            if constexpr (sizeof(Tc) == 4) {
+                const float4 c4 = *reinterpret_cast<const float4*>(rowC + 4 * er);
+                w.cN = c4.x; w.cS = c4.y; w.cF = c4.z; w.cB = c4.w;
+            } else {
+                const double2 a2 = *reinterpret_cast<const double2*>(rowC + 4 * er);
+                const double2 b2 = *reinterpret_cast<const double2*>(rowC + 4 * er + 2);
+                w.cN = a2.x; w.cS = a2.y; w.cF = b2.x; w.cB = b2.y;
+            }
             w.par = rt.w;
-            w.gr = rt.z;
+            if (EDGE) {
+                const int2 pb = pubT[er];
+                w.pubA = pb.x >= 0 ? Ec + (size_t)pb.x * Word::n : nullptr;
+                w.pubB = pb.y >= 0 ? Ec + (size_t)pb.y * Word::n : nullptr;
+            }
             return w;
         };
-        using I0 = std::integral_constant<int, 0>;
-        using I1 = std::integral_constant<int, 1>;
         if constexpr (MODE == kResNarrow) {
-            // two rows per warp, lane t in each
-            for (int er = e0r + 2 * warp; er < e1r; er += 2 * NWARP) {
-                const bool twoRows = er + 1 < e1r;
-                const ResRow<Tc> wA = row_of(er), wB = row_of(twoRows ? er + 1 : er);
+            // rows of at most 32 cells per colour: a warp takes 2 rpw rows at a time, rpw side by
+            // side over the lanes (rpw = 32 / nown1), twice
+            for (int er = e0r + 2 * rpw * warp + sub; er < e1r + sub; er += 2 * rpw * NWARP) {
+                const int eB = er + rpw;
+                const bool inA = sub < rpw && er < e1r, inB = sub < rpw && eB < e1r;
+                const ResRow<Tc> wA = row_of(inA ? er : e0r), wB = row_of(inB ? eB : e0r);
                 const int rA = (wA.par ^ c) & 1, rB = (wB.par ^ c) & 1;
-                const bool okA = lane < (rA ? nown1 : nown0);
-                const bool okB = twoRows && lane < (rB ? nown1 : nown0);
-                auto two = [&](auto ra, auto rb) {
-                    constexpr int RA = decltype(ra)::value, RB = decltype(rb)::value;
-                    const int mA = lane + 2 - RA, mB = lane + 2 - RB;
-                    const ResIn<Tc> xA = res_load<Tc, CD, CR, RA>(wA, mA, mx, plane);
-                    const ResIn<Tc> xB = res_load<Tc, CD, CR, RB>(wB, mB, mx, plane);
-                    res_finish<Tc, EDGE>(xA, wA, mA, cEr[RA][0], cWr[RA][0], om, okA, Ec, ch);
-                    res_finish<Tc, EDGE>(xB, wB, mB, cEr[RB][0], cWr[RB][0], om, okB, Ec, ch);
-                };
-                if (rA == 0) {
-                    if (rB == 0) two(I0{}, I0{});
-                    else two(I0{}, I1{});
-                } else {
-                    if (rB == 0) two(I1{}, I0{});
-                    else two(I1{}, I1{});
-                }
+                const int mA = lt + 2 - rA, mB = lt + 2 - rB;
+                const ResIn<Tc> xA = res_load<Tc, CD, CR>(wA, lt, mA, mx, plane);
+                const ResIn<Tc> xB = res_load<Tc, CD, CR>(wB, lt, mB, mx, plane);
+                res_finish<Tc, EDGE>(xA, wA, lt, mA, rA ? cEr[1][0] : cEr[0][0], rA ? cWr[1][0] : cWr[0][0], om,
+                                     inA && lt < (rA ? nown1 : nown0), inA, seq, ch);
+                res_finish<Tc, EDGE>(xB, wB, lt, mB, rB ? cEr[1][0] : cEr[0][0], rB ? cWr[1][0] : cWr[0][0], om,
+                                     inB && lt < (rB ? nown1 : nown0), inB, seq, ch);
             }
         } else {
             for (int er = e0r + warp; er < e1r; er += NWARP) {
                 const ResRow<Tc> w = row_of(er);
                 const int r = (w.par ^ c) & 1;
                 const int nown = r ? nown1 : nown0;
-                auto one = [&](auto rr) {
-                    constexpr int R = decltype(rr)::value;
-                    if constexpr (MODE == kResWide1) {
-                        // cells t = lane (always in the row: it holds more than 32) and lane + 32
-                        const int mA = lane + 2 - R;
-                        const ResIn<Tc> xA = res_load<Tc, CD, CR, R>(w, mA, mx, plane);
-                        const ResIn<Tc> xB = res_load<Tc, CD, CR, R>(w, mA + 32, mx, plane);
-                        res_finish<Tc, EDGE>(xA, w, mA, cEr[R][0], cWr[R][0], om, true, Ec, ch);
-                        res_finish<Tc, EDGE>(xB, w, mA + 32, cEr[R][1], cWr[R][1], om, lane + 32 < nown, Ec, ch);
-                    } else {
-                        for (int t0 = 0; t0 < nown; t0 += 64) {
-                            const int tA = t0 + lane;
-                            const int mA = tA + 2 - R;
-                            const ResIn<Tc> xA = res_load<Tc, CD, CR, R>(w, mA, mx, plane);
-                            const ResIn<Tc> xB = res_load<Tc, CD, CR, R>(w, mA + 32, mx, plane);
-                            const int iA = min(2 * tA + 2 - R, g.nx + 2), iB = min(iA + 64, g.nx + 2);
-                            const Tc eA = cEs[iA], wA = cWs[iA], eB = cEs[iB], wB = cWs[iB];
-                            res_finish<Tc, EDGE>(xA, w, mA, eA, wA, om, tA < nown, Ec, ch);
-                            res_finish<Tc, EDGE>(xB, w, mA + 32, eB, wB, om, tA + 32 < nown, Ec, ch);
-                        }
+                if constexpr (MODE == kResWide1) {
+                    // cells t = lane (always in the row: it holds more than 32) and lane + 32
+                    const int m = lane + 2 - r;
+                    const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, lane, m, mx, plane);
+                    const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, lane + 32, m + 32, mx, plane);
+                    res_finish<Tc, EDGE>(xA, w, lane, m, r ? cEr[1][0] : cEr[0][0], r ? cWr[1][0] : cWr[0][0], om, true, true,
+                                         seq, ch);
+                    res_finish<Tc, EDGE>(xB, w, lane + 32, m + 32, r ? cEr[1][1] : cEr[0][1], r ? cWr[1][1] : cWr[0][1], om,
+                                         lane + 32 < nown, lane + 32 < nown1, seq, ch);
+                } else {
+                    for (int t0 = 0; t0 < nown1; t0 += 64) {
+                        const int tA = t0 + lane, m = tA + 2 - r;
+                        const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, tA, m, mx, plane);
+                        const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, tA + 32, m + 32, mx, plane);
+                        const int iA = min(2 * tA + 2 - r, g.nx + 2), iB = min(iA + 64, g.nx + 2);
+                        const Tc eA = cEs[iA], wA = cWs[iA], eB = cEs[iB], wB = cWs[iB];
+                        res_finish<Tc, EDGE>(xA, w, tA, m, eA, wA, om, tA < nown, tA < nown1, seq, ch);
+                        res_finish<Tc, EDGE>(xB, w, tA + 32, m + 32, eB, wB, om, tA + 32 < nown, tA + 32 < nown1, seq, ch);
                     }
-                };
-                if (r == 0) one(I0{});
-                else one(I1{});
+                }
             }
         }
     };
     using EdgeT = std::integral_constant<bool, true>;
     using InnerT = std::integral_constant<bool, false>;
 
+    // a change above zeta, NaN included: FP32 changes against the largest float <= zeta
+    const float zf = __double2float_rd(zeta);
+    auto above = [&](B ch) {
+        if constexpr (sizeof(Tc) == 4) return !(__uint_as_float(ch) <= zf);
+        else return !(__longlong_as_double((long long)ch) <= zeta);
+    };
+    auto verdict = [&](int any, int par) {
+        return 1ull | (unsigned long long)((any ? 1u : 0u) + (s_nan[par] ? kNanFlag : 0u)) << 32;
+    };
+    constexpr B kInf = sizeof(Tc) == 4 ? (B)0x7f800000u : (B)kInfBits;
+
   for (;;) {
-    if (failed) break;
     done_c = 0;
+#pragma unroll 1
     for (int s = 0; ik0 + done + s < itmax && s < cycle_len; ++s) {
-        const int sg = done + s;   // sweep of this launch: ring slot
-        if (blockIdx.x == 0 && tid == 0) ring[(sg + 1) % 3] = 0ULL;
-        B ch = B(0);
-        Tc fv[kFill];
-        // red half: the black ring in flight (it is 0 in a cycle's first sweep), the
-        // interior rows, the ring, the edge rows (published), arrive
-        if (s > 0) fill_issue(0, fv);
-        rows_pass(InnerT{}, 0, ne, nrows, ch);
-        if (s > 0) fill_commit(0, fv);
-        rows_pass(EdgeT{}, 0, 0, ne, ch);
-        grid_arrive(bar, nbar);
-        // black half: the interior rows (they read only this brick's red values) while
-        // the barrier completes, wait, the red ring, the edge rows (published), then this
-        // CTA's max |change| over the sweep into the ring slot of sweep sg and a full
-        // barrier, so that every CTA's max is in the ring before anyone reads it
-        rows_pass(InnerT{}, 1, ne, nrows, ch);
-        if (!grid_wait(bar, nbar, nblocks, &s_flag)) {
+        const int sg = done + s, par = sg & 1;      // sweep of this launch
+        const unsigned int target = nblocks * (unsigned)((sg >> 2) + 1);
+        const int ik = ik0 + sg + 1;
+        const bool test = check_every == 1 || ik >= itmax || ik % check_every == 0;
+        B ch = B(0);                                // over both colours
+        unsigned int vr = 0u, vb = 0u;              // verdicts: CTAs with a red, a black change above zeta
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            const unsigned int seq = seq0 + 2u * (unsigned)sg + 1u + (unsigned)c;
+            B cc = B(0);
+            // the interior rows read only this brick's values; the ring (0 in a cycle's first
+            // half-sweep), the edge rows (published)
+            rows_pass(InnerT{}, c, ne, nrows, seq, cc);
+            if (multi) {
+                if (c || s > 0) fill(1 - c, seq - 1u, par);
+                __syncthreads();
+                if (s_fail[par]) {
+                    failed = true;
+                    break;
+                }
+            }
+            // the counters' first look, a trip through L2 ahead of its use
+            unsigned long long wr = 0ull, wb = 0ull;
+            if (c && ctrl) {
+                wr = ld_relaxed(&sync->cnt[0][sg & 3]);
+                wb = ld_relaxed(&sync->cnt[1][(sg + 3) & 3]);
+            }
+            rows_pass(EdgeT{}, c, 0, ne, seq, cc);
+            if (cc >= kInf) s_nan[par] = 1;
+            if (c && ctrl) {
+                // the red half's verdicts, and whether the sweep before met a NaN in its black half
+                if ((int)((unsigned int)wr - target) < 0 &&
+                    !count_wait(&sync->cnt[0][sg & 3], target, &sync->bar.err, &wr))
+                    s_fail[par] = 1;
+                const unsigned int h0 = (unsigned int)(wr >> 32), h1 = (unsigned int)(wb >> 32);
+                s_vd = make_uint2(h0 - s_prev[0][sg & 3], sg > 0 ? h1 - s_prev[1][(sg + 3) & 3] : 0u);
+                s_prev[0][sg & 3] = h0;
+                if (sg > 0) s_prev[1][(sg + 3) & 3] = h1;
+            }
+            const int any = __syncthreads_or(above(cc));
+            if (ctrl) red_add_relaxed(&sync->cnt[c][sg & 3], verdict(any, par));
+            (c ? vb : vr) = any ? 1u : 0u;
+            ch = cc > ch ? cc : ch;
+        }
+        if (failed) break;
+        if (s_fail[par]) {
             failed = true;
             break;
         }
-        fill_issue(1, fv);
-        fill_commit(1, fv);
-        rows_pass(EdgeT{}, 1, 0, ne, ch);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const B t2 = __shfl_xor_sync(0xffffffffu, ch, o);
-            ch = t2 > ch ? t2 : ch;
+        if (multi) {
+            const uint2 vd = s_vd;
+            if (prev_tested && vd.y >= kNanFlag) {
+                nonfinite = true;                   // met in the sweep before
+                break;
+            }
+            vr = vd.x;
+        } else if (s_nan[par]) {
+            vr = kNanFlag;
         }
-        if (lane == 0) s_red[warp] = ch;
-        __syncthreads();
-        // the CTA's max: whether it is above zeta (or not finite) rides on this CTA's
-        // arrival at the closing barrier; the value itself goes to the ring slot of
-        // the sweep after the arrival, off the critical path (the solve's last one is
-        // read after a final barrier)
-        unsigned long long mybits = 0ull;
-        unsigned int flags = 0u;
-        if (tid == 0) {
-            B b2 = B(0);
-            for (int q = 0; q < NWARP; ++q) b2 = s_red[q] > b2 ? s_red[q] : b2;
-            mybits = widen_bits(b2);
-            flags = (mybits >= kInfBits ? kNanFlag : 0u) |
-                    ((__longlong_as_double((long long)mybits) > zeta || mybits >= kInfBits) ? 1u : 0u);
-        }
-        grid_arrive(bar, nbar, flags);
-        if (tid == 0 && mybits != 0ull) atomicMax(&ring[sg % 3], mybits);
-        if (!grid_wait(bar, nbar, nblocks, &s_flag, &s_hi)) {
-            failed = true;
-            break;
-        }
-        const unsigned int over = s_hi - hi_prev;   // CTAs above zeta, + kNanFlag per non-finite one
-        hi_prev = s_hi;
+        chs = ch;
         done_c = s + 1;
-        const int ik = ik0 + done + done_c;
-        if (ik % check_every == 0 || ik >= itmax) {
-            nonfinite = over >= kNanFlag;
-            conv = over == 0u;
+        prev_tested = test;
+        if (test) {
             tested = true;
+            if (multi && vr < kNanFlag && (vr == 0u || ik >= itmax)) {
+                __syncthreads();                    // s_vd has been read
+                if (ctrl) {
+                    unsigned long long w = 0ull;
+                    if (!count_wait(&sync->cnt[1][sg & 3], target, &sync->bar.err, &w)) s_fail[par] = 1;
+                    s_vd.y = (unsigned int)(w >> 32) - s_prev[1][sg & 3];
+                }
+                __syncthreads();
+                if (s_fail[par]) {
+                    failed = true;
+                    break;
+                }
+                vb = s_vd.y;
+            }
+            nonfinite = vr >= kNanFlag || vb >= kNanFlag;
+            conv = vr == 0u && vb == 0u;
             if (conv || nonfinite) break;
         }
     }
     done += done_c;
     // another cycle only when this one ended on its length
     if (failed || conv || nonfinite || done_c < cycle_len || ik0 + done >= itmax) break;
-    // restart: the black ring again (the neighbours' final black rows; the red one is
-    // current), d = the FP64 defect of p + e and p += e in one pass, e = 0.  No grid barrier: the
-    // next cycle's first red half reads a zero black ring, and its black half reads
-    // red rows published after the next barrier.
-    {
-        Tc fv[kFill];
-        fill_issue(0, fv);
-        fill_commit(0, fv);
+    // restart: the black ring once more (the neighbours' final black rows; the red one is
+    // current), d = the FP64 defect of p + e and p += e in one pass, e = 0
+    if (multi) {
+        fill(1, seq0 + 2u * (unsigned)done, done & 1);
+        __syncthreads();
+        if (s_fail[done & 1]) {
+            failed = true;
+            break;
+        }
     }
     update_defect();
     __syncthreads();
@@ -644,11 +711,29 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     ++restarts;
   }
     add_e_to_p();
-    // the max |change| of the last (tested) sweep, whose slot every CTA has reached
-    // through the release of a later arrival
-    if (!failed && tested && done > 0 && grid_sync(bar, nbar, nblocks, &s_flag) && tid == 0)
-        last = __longlong_as_double((long long)*(const volatile unsigned long long*)&ring[(done - 1) % 3]);
+    // the max |change| of the last (tested) sweep
+    if (!failed && tested && done > 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const B t2 = __shfl_xor_sync(0xffffffffu, chs, o);
+            chs = t2 > chs ? t2 : chs;
+        }
+        if (lane == 0) s_red_max[warp] = chs;
+        __syncthreads();
+        if (tid == 0) {
+            B b2 = B(0);
+            for (int q = 0; q < NWARP; ++q) b2 = s_red_max[q] > b2 ? s_red_max[q] : b2;
+            if (multi) atomicMax(&sync->last, widen_bits(b2));
+            else last = __longlong_as_double((long long)widen_bits(b2));
+        }
+        if (multi) {
+            unsigned int nbar = 0;
+            if (!grid_sync(&sync->bar, nbar, nblocks, &s_flag)) failed = true;
+            else if (tid == 0) last = __longlong_as_double((long long)ld_relaxed(&sync->last));
+        }
+    }
     if (blockIdx.x == 0 && tid == 0) {
+        sync->seq = seq0 + (failed ? 1u << 24 : 2u * (unsigned)done + 4u);
         ctl->ik = ik0 + done;
         ctl->inner = done_c;
         ctl->cycles += restarts + (itmax > 0 ? 1 : 0);   // the launch's cycles, the last included

@@ -115,8 +115,9 @@ struct ntcfd_ctx {
     int rec_host_cap = 0;
     unsigned long long* slots = nullptr;   // per-sweep max |change| bits
     unsigned long long* divslot = nullptr;
-    GridBar* bar = nullptr;                 // grid barrier of the resident SOR kernel
-    unsigned long long* ring = nullptr;     // its per-sweep max |change| ring
+    ResSync* rsync = nullptr;               // counters of the resident SOR kernel
+    unsigned long long* boxes = nullptr;    // its inboxes (made with the first plan, kept)
+    size_t box_words = 0;
     Brick brick{};
     bool resident = false;                  // the graph uses the resident SOR kernel
     size_t res_smem = 0;
@@ -342,8 +343,8 @@ SorCoef<float> sor_coef<float>(ntcfd_ctx* ctx) { return ctx->scf; }
 
 // The resident SOR kernel for a brick plan (d and rd cached or not, row shape).
 template <class Tc>
-using ResidentFn = void (*)(Geom, SorCoef<Tc>, Brick, double*, const double*, Tc*, Tc*, Tc*, Tc*, const Tc*,
-                            const Tc*, Ctl*, GridBar*, double, double, int, int, int, unsigned long long*);
+using ResidentFn = void (*)(Geom, SorCoef<Tc>, Brick, double*, const double*, Tc*, Tc*, const Tc*, const Tc*, Ctl*,
+                            ResSync*, unsigned long long*, double, double, int, int, int);
 template <class Tc, int MODE>
 ResidentFn<Tc> resident_kernel_m(const Brick& b) {
     if (b.cache_d && b.cache_rd) return k_sor_resident<Tc, kResNT, true, true, MODE>;
@@ -359,36 +360,44 @@ ResidentFn<Tc> resident_kernel(const Brick& b) {
 }
 
 // Brick plan of the resident SOR kernel: the split of the (j,k) rows into at
-// most (SM count) bricks that minimises the largest brick, under the shared
+// most (SM count) bricks of least estimated time per half-sweep, under the shared
 // memory limit (e of both colours for the brick and a one-row halo, plus d
-// when it also fits).  Returns false when no plan fits one CTA per SM.
+// when it also fits).  Bricks with a neighbour are two rows thick or more.
+// The estimate, in clocks: a pass of the warps over the interior rows takes about
+// 360 (one row a warp; 640 for the narrow form's two slots, each of several rows),
+// over the edge rows, which publish, 1.6 times that, FP64 1.7 times more (twice the
+// shared-memory words); rows without cached d and rd half as much again; the
+// hand-over between CTAs 1500.  So a grid of few rows runs in one CTA without any
+// hand-over: 12x10x8 takes 2.0 us a sweep (FP32) and 2.3 us (FP64) there against
+// 3.2 and 3.0 on 4 CTAs.  Returns false when no plan fits one CTA per SM.
 template <class Tc>
 bool plan_resident(ntcfd_ctx* ctx) {
     const Geom& g = ctx->g;
-    const int mx = ((g.nx + 3) >> 1) + 1;
+    const int mx = ((g.nx + 3) >> 1) + 1, half = (g.nx + 1) / 2;
     const size_t limit = ctx->smem_optin > 4096 ? ctx->smem_optin - 4096 : 0;
-    long long best = -1;
+    const int mode = res_mode(g.nx);
+    const long long per = kResNT / 32 * (mode == kResNarrow ? 2 * (32 / half) : 1);   // rows of a pass
+    const double pass = (mode == kResNarrow ? 640.0 : 360.0 * ((half + 63) / 64)) * (sizeof(Tc) == 8 ? 1.7 : 1.0);
+    double best = -1.0;
     Brick bb{};
     size_t bsm = 0;
-    for (int nbk = 1; nbk <= g.nz; ++nbk) {
+    for (int nbk = 1; nbk <= std::max(1, g.nz / 2) && nbk <= ctx->sm_count; ++nbk) {
         const int KB = (g.nz + nbk - 1) / nbk;
-        const int nbk_eff = (g.nz + KB - 1) / KB;
-        for (int nbj = 1; nbj <= g.ny; ++nbj) {
+        for (int nbj = 1; nbj <= std::max(1, g.ny / 2) && nbj * nbk <= ctx->sm_count; ++nbj) {
             const int JB = (g.ny + nbj - 1) / nbj;
-            const int nbj_eff = (g.ny + JB - 1) / JB;
-            if ((long long)nbj_eff * nbk_eff > ctx->sm_count) continue;
-            Brick b{nbj_eff, nbk_eff, JB, KB, mx, 0, 0, res_mode(g.nx)};
+            Brick b{nbj, nbk, JB, KB, mx, 0, 0, mode, 2 * (JB + KB) * half};
             if (resident_smem<Tc>(b, g.nx) > limit) continue;
             // cache d, then rd, when they fit as well
             b.cache_d = 1;
             if (resident_smem<Tc>(b, g.nx) > limit) b.cache_d = 0;
             b.cache_rd = 1;
             if (resident_smem<Tc>(b, g.nx) > limit) b.cache_rd = 0;
-            const long long cells = (long long)JB * KB;
-            // smallest brick first, then the more cached arrays, then the smaller halo
-            const long long score = cells * 1000000LL + (2 - b.cache_d - b.cache_rd) * 10000LL + (JB + KB);
-            if (best < 0 || score < best) {
-                best = score;
+            const long long rows = (long long)JB * KB, ni = JB > 2 && KB > 2 ? (long long)(JB - 2) * (KB - 2) : 0;
+            const double cost = pass * (double)((ni + per - 1) / per + 1.6 * ((rows - ni + per - 1) / per)) *
+                                    (1.0 + 0.25 * (2 - b.cache_d - b.cache_rd)) +
+                                (nbj * nbk > 1 ? 1500.0 : 300.0) + 0.01 * (JB + KB);
+            if (best < 0 || cost < best) {
+                best = cost;
                 bb = b;
                 bsm = resident_smem<Tc>(b, g.nx);
             }
@@ -405,6 +414,11 @@ bool plan_resident(ntcfd_ctx* ctx) {
         per_sm < 1 || (long long)bb.nbj * bb.nbk > (long long)per_sm * ctx->sm_count) {
         cudaGetLastError();
         return false;
+    }
+    const size_t words = (size_t)bb.nbj * bb.nbk * 2 * bb.inbox * RingWord<Tc>::n;
+    if (words > ctx->box_words) {
+        if (dalloc(ctx, &ctx->boxes, words)) return false;
+        ctx->box_words = words;
     }
     ctx->brick = bb;
     ctx->res_smem = bsm;
@@ -484,12 +498,12 @@ int add_step_nodes(ntcfd_ctx* ctx, cudaGraph_t G, int extra) {
         Tc *eR = (Tc*)ctx->eR, *eB = (Tc*)ctx->eB, *dR = (Tc*)ctx->dR, *dB = (Tc*)ctx->dB;
         GK(add_kernel(&n, G, dep, k_defect<Tc>, g3, b3, g, ctx->scd, (const double*)ctx->p,
                       (const double*)ctx->b, dR, dB, eR, eB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl,
-                      (cudaGraphConditionalHandle)0, 0, ctx->ring, (unsigned int*)ctx->bar, 1, 0));
+                      (cudaGraphConditionalHandle)0, 0, ctx->rsync, 1, 0));
         dep = {n};
         GK(add_kernel_ex(&n, G, dep, resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT),
                          ctx->res_smem, true, g, sor_coef<Tc>(ctx), ctx->brick, ctx->p, (const double*)ctx->b,
-                         eR, eB, dR, dB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl,
-                         ctx->bar, P.omega, P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps, ctx->ring));
+                         dR, dB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, ctx->rsync, ctx->boxes, P.omega,
+                         P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps));
         dep = {n};
     } else {
         cudaGraphConditionalHandle hout, hin;
@@ -673,11 +687,10 @@ int sor_solve_eager(ntcfd_ctx* ctx, double* p, const double* b, double zeta, int
     if (ctx->resident) {
         // one defect (starting the solve) and one launch that runs every cycle
         k_defect<Tc><<<g3, b3, 0, st>>>(g, ctx->scd, p, b, dR, dB, eR, eB, (const Tc*)ctx->rdR,
-                                        (const Tc*)ctx->rdB, ctx->ctl, 0, 0, ctx->ring, (unsigned int*)ctx->bar, 1, 0);
-        void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&p, (void*)&b, (void*)&eR,
-                        (void*)&eB, (void*)&dR, (void*)&dB, (void*)&ctx->rdR, (void*)&ctx->rdB,
-                        (void*)&ctx->ctl, (void*)&ctx->bar, (void*)&omega, (void*)&zeta,
-                        (void*)&itmax, (void*)&ctx->cycle_len, (void*)&ctx->csweeps, (void*)&ctx->ring};
+                                        (const Tc*)ctx->rdB, ctx->ctl, 0, 0, ctx->rsync, 1, 0);
+        void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&p, (void*)&b, (void*)&dR, (void*)&dB,
+                        (void*)&ctx->rdR, (void*)&ctx->rdB, (void*)&ctx->ctl, (void*)&ctx->rsync, (void*)&ctx->boxes,
+                        (void*)&omega, (void*)&zeta, (void*)&itmax, (void*)&ctx->cycle_len, (void*)&ctx->csweeps};
         CK(cudaLaunchCooperativeKernel((const void*)resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid),
                                        dim3(kResNT), args, ctx->res_smem, st));
         if (int rc = read_ctl()) return rc;
@@ -866,7 +879,7 @@ int time_kernels_t(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
              if (ctx->resident)
                  k_defect<Tc><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, ctx->p, ctx->b, dR, dB, eR, eB,
                                                           (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, 0, 0,
-                                                          nullptr, nullptr, 0, 0);
+                                                          nullptr, 0, 0);
              else
                  // on scratch (us is rewritten by the predictor every step): from a
                  // cycle on, the restart also adds e to the p it is given
@@ -896,11 +909,11 @@ int time_kernels_t(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
         auto resident = [&](const int* sweeps) {
             k_defect<Tc><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, pscratch, ctx->b, dR, dB, eR, eB,
                                                      (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, 0, 0,
-                                                     ctx->ring, (unsigned int*)ctx->bar, 1, 0);
-            void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&pscratch, (void*)&ctx->b,
-                            (void*)&eR, (void*)&eB, (void*)&dR, (void*)&dB, (void*)&ctx->rdR, (void*)&ctx->rdB,
-                            (void*)&ctx->ctl, (void*)&ctx->bar, (void*)&P.omega, (void*)&kZeroZeta,
-                            (void*)sweeps, (void*)sweeps, (void*)&kOne, (void*)&ctx->ring};
+                                                     ctx->rsync, 1, 0);
+            void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&pscratch, (void*)&ctx->b, (void*)&dR,
+                            (void*)&dB, (void*)&ctx->rdR, (void*)&ctx->rdB, (void*)&ctx->ctl, (void*)&ctx->rsync,
+                            (void*)&ctx->boxes, (void*)&P.omega, (void*)&kZeroZeta, (void*)sweeps, (void*)sweeps,
+                            (void*)&kOne};
             cudaLaunchCooperativeKernel((const void*)resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid),
                                         dim3(kResNT), args, ctx->res_smem, ctx->stream);
         };
@@ -1033,8 +1046,7 @@ int ntcfd_create(const ntcfd_params* prm, ntcfd_ctx** out) {
     if ((rc = dalloc(ctx, &ctx->ctl, 1))) return rc;
     if ((rc = dalloc(ctx, &ctx->slots, 64 * kSpread))) return rc;
     if ((rc = dalloc(ctx, &ctx->divslot, 1))) return rc;
-    if ((rc = dalloc(ctx, &ctx->bar, 1))) return rc;
-    if ((rc = dalloc(ctx, &ctx->ring, 4))) return rc;
+    if ((rc = dalloc(ctx, &ctx->rsync, 1))) return rc;
     {
         int v = 0;
         CK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, P.device));
@@ -1648,7 +1660,7 @@ int ntcfd_slab_stage(ntcfd_ctx* ctx, int stage, int colour) {
             k_sor_begin<<<1, 1, 0, st>>>(ctx->ctl, P.itmax, 0, 0);
             k_defect<double><<<g3, b3, 0, st>>>(g, ctx->scd, ctx->p, ctx->b, dR, dB, eR, eB,
                                                 (const double*)ctx->rdR, (const double*)ctx->rdB, ctx->ctl, 0, 0,
-                                                nullptr, nullptr, 0, 0);
+                                                nullptr, 0, 0);
             k_clear_e<double><<<g3, b3, 0, st>>>(g, eR, eB);
             // the ghost planes of e hold the neighbours' last planes of the previous
             // solve: theirs start from zero too
