@@ -296,7 +296,7 @@ def roofline(s, case, path, reps=20):
         alg = 3 * S * N * kt["resident_sweeps"]
         ms = kt["resident_ms"]
     else:
-        kernel = "k_sweep (one colour of a red-black SOR sweep)"
+        kernel = "k_sor_march, or k_sweep of wide rows (half a red-black SOR sweep)"
         alg = 1.5 * S * N
         ms = kt["sweep_ms"]
     ach = alg / (ms * 1e-3) / 1e9

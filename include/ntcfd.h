@@ -62,12 +62,14 @@ enum { NTCFD_QUICK_CENTRE = 0, NTCFD_QUICK = 1, NTCFD_UPWIND = 2, NTCFD_CENTRE =
 enum { NTCFD_SMAG_REF_ALIASED = 0, NTCFD_SMAG_STAGGERED = 1 };
 enum { NTCFD_SOR_REDBLACK = 0, NTCFD_SOR_LEX = 1 };    /* LEX: oracle only */
 /* How the sweeps of one correction cycle run on the device:
- * STREAMING -- two kernels per sweep (one per colour) reading e from
- *              global memory, the loop driven by CUDA-graph conditional nodes;
- * RESIDENT  -- one persistent cooperative kernel per cycle with e kept in
+ * STREAMING -- e in global memory: one persistent cooperative kernel that
+ *              marches through the planes (rows of up to 234 cells), or two
+ *              kernels per sweep (one per colour), the loop driven by
+ *              CUDA-graph conditional nodes;
+ * RESIDENT  -- one persistent cooperative kernel per solve with e kept in
  *              shared memory (only when the grid's e fits on the chip);
- * AUTO      -- RESIDENT when it fits, else STREAMING.  Both run the same
- *              red-black iteration and stop rule. */
+ * AUTO      -- RESIDENT when it fits and is the faster, else STREAMING.  All
+ *              run the same red-black iteration and stop rule. */
 enum { NTCFD_SOR_AUTO = 0, NTCFD_SOR_STREAMING = 1, NTCFD_SOR_RESIDENT = 2 };
 
 typedef struct ntcfd_params {
@@ -115,7 +117,7 @@ typedef struct ntcfd_kernel_times {
     float predictor_ms;      /* K2 (with K1 when LES = 1), one launch */
     float rhs_ms;            /* K3a */
     float defect_ms;         /* defect pass of a correction cycle */
-    float sweep_ms;          /* one half-sweep (one colour) */
+    float sweep_ms;          /* one half-sweep (one colour; half a sweep of the marching kernel) */
     float project_ms;        /* K4, measured on a copy of the velocity */
     float bc_ms;             /* the three K6 launches together */
     float resident_ms;       /* one resident-SOR launch running resident_sweeps sweeps (0 if unused) */
