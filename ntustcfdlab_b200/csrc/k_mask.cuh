@@ -13,138 +13,180 @@
 
 namespace ntcfd {
 
-// ETA_1 from the crossing parity (airfoil.f90:685-764) of cell (k,j).
-// Y, Z: node coordinates pre-offset (Y[j] valid for j in -1..n+3).
-__device__ __forceinline__ void ray_main_cell(int k, int j, int nz, const double* Y, const double* Z,
-                                              const double* az, const double* ay, int poly, double* eta1,
-                                              int* ties) {
-    const double Yj = Y[j], Zk = Z[k];
-    const double ycell = (Y[j] + Y[j + 1]) / 2.0;
-    const double zcell = (Z[k] + Z[k + 1]) / 2.0;
-    int cnt = 0, tie = 0;
-    for (int m = 0; m < poly - 1; ++m) {
-        const double a0 = ay[m], a1 = ay[m + 1], z0 = az[m], z1 = az[m + 1];
-        if (a0 >= ycell && a1 <= ycell) {
-            if (zcell >= fmax(z0, z1)) {
-            } else if (zcell < fmin(z0, z1)) {
-                ++cnt;
-            } else {
-                if (Yj == a1 || Zk == z1) ++tie;
-                const double m_pa = (Yj - a1) / (Zk - z1);
-                const double m_ab = (a0 - a1) / (z0 - z1);
-                if (m_pa > m_ab) ++cnt;
+// A list of polygon edges in shared memory, filled by the block NT edges at a time.
+template <int NT>
+struct EdgeList {
+    double a0[NT], a1[NT], z0[NT], z1[NT];           // ay, az of the edge's ends
+    int count[2];                                    // listed of this pass, and of the next
+    // Lists the edges m0 .. m0 + NT - 1 that `keep` takes; every thread of the block.
+    template <class Keep>
+    __device__ __forceinline__ int fill(int m0, int pass, const double* az, const double* ay, int poly, Keep&& keep) {
+        const int m = m0 + threadIdx.x;
+        if (m < poly - 1) {
+            const double p0 = ay[m], p1 = ay[m + 1], q0 = az[m], q1 = az[m + 1];
+            if (keep(p0, p1, q0, q1)) {
+                const int e = atomicAdd(&count[pass], 1);
+                a0[e] = p0; a1[e] = p1; z0[e] = q0; z1[e] = q1;
             }
         }
-        if (a0 <= ycell && a1 >= ycell) {
-            if (zcell >= fmax(z0, z1)) {
-            } else if (zcell < fmin(z0, z1)) {
-                ++cnt;
-            } else {
-                if (Yj == a0 || Zk == z0) ++tie;
-                const double m_pa = (Yj - a0) / (Zk - z0);
-                const double m_ab = (a1 - a0) / (z1 - z0);
-                if (m_pa > m_ab) ++cnt;
-            }
-        }
+        if (threadIdx.x == 0) count[pass ^ 1] = 0;
+        __syncthreads();
+        return count[pass];
     }
-    eta1[(long long)(k - 1) + (long long)nz * (j - 1)] = (cnt % 2 == 0) ? 0.0 : 1.0;
+};
+
+// ETA_1 of the cells k of row j from their crossing parity (airfoil.f90:685-764), a thread
+// per cell.  Y, Z: node coordinates pre-offset (Y[j] valid for j in -1..n+3).
+//
+// Only edges that span the row's cell centres count, so the block lists those (some 2 to 30 of
+// 511 for an airfoil) and its threads test the list: 64x192x256 6 us against
+// 73 us with every cell testing every edge from memory.
+template <int NT>
+__device__ __forceinline__ void ray_main_row(int k, int j, int nz, const double* Y, const double* Z,
+                                             const double* az, const double* ay, int poly, double* eta1,
+                                             int* ties, EdgeList<NT>& ed) {
+    const double Yj = Y[j], ycell = (Y[j] + Y[j + 1]) / 2.0;
+    const bool in = k <= nz;
+    const double Zk = in ? Z[k] : 0.0, zcell = in ? (Z[k] + Z[k + 1]) / 2.0 : 0.0;
+    int cnt = 0, tie = 0;
+    if (threadIdx.x == 0) ed.count[0] = 0;
+    __syncthreads();
+    for (int m0 = 0, pass = 0; m0 < poly - 1; m0 += NT, pass ^= 1) {
+        const int count = ed.fill(m0, pass, az, ay, poly, [&](double a0, double a1, double, double) {
+            return (a0 >= ycell && a1 <= ycell) || (a0 <= ycell && a1 >= ycell);
+        });
+        for (int e = 0; in && e < count; ++e) {
+            const double a0 = ed.a0[e], a1 = ed.a1[e], z0 = ed.z0[e], z1 = ed.z1[e];
+            const bool down = a0 >= ycell && a1 <= ycell, up = a0 <= ycell && a1 >= ycell;
+            if (zcell >= fmax(z0, z1)) continue;
+            if (zcell < fmin(z0, z1)) {
+                cnt += (down ? 1 : 0) + (up ? 1 : 0);
+                continue;
+            }
+            if (down) {
+                if (Yj == a1 || Zk == z1) ++tie;
+                if ((Yj - a1) / (Zk - z1) > (a0 - a1) / (z0 - z1)) ++cnt;
+            }
+            if (up) {
+                if (Yj == a0 || Zk == z0) ++tie;
+                if ((Yj - a0) / (Zk - z0) > (a1 - a0) / (z1 - z0)) ++cnt;
+            }
+        }
+        __syncthreads();                             // the list is read
+    }
+    if (in) eta1[(long long)(k - 1) + (long long)nz * (j - 1)] = (cnt % 2 == 0) ? 0.0 : 1.0;
     if (tie) atomicAdd(ties, tie);
 }
 
-__global__ void k_ray_main(int ny, int nz, const double* Y, const double* Z, const double* az,
-                           const double* ay, int poly, double* eta1, int* ties) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    if (k > nz || j > ny) return;
-    ray_main_cell(k, j, nz, Y, Z, az, ay, poly, eta1, ties);
-}
-
-// points(k,j) = 1 when a polygon vertex lies in [Z(k),Z(k+1)) x [Y(j),Y(j+1))
-// for k in C..E-1, j in A..B-1 (airfoil.f90:661-674).
+// The cell that holds polygon vertex m, in [Z(k),Z(k+1)) x [Y(j),Y(j+1)) for k in C..E-1, j in
+// A..B-1 (airfoil.f90:661-674): flagged and, by the first vertex found in it, listed.  One
+// warp per vertex (a thread per vertex walks the nodes one load after another: 34 us
+// for 512 vertices on 192x256 nodes, 6 us by warps).
 __device__ __forceinline__ void ray_point(int m, int ny, int nz, const double* Y, const double* Z,
                                           const double* az, const double* ay, int A, int B, int C, int E,
-                                          int* points) {
-    for (int k = C; k <= E - 1; ++k) {
-        if (!(az[m] >= Z[k] && az[m] < Z[k + 1])) continue;
-        for (int j = A; j <= B - 1; ++j)
-            if (ay[m] >= Y[j] && ay[m] < Y[j + 1] && k >= 1 && k <= nz && j >= 1 && j <= ny)
-                points[(long long)(k - 1) + (long long)nz * (j - 1)] = 1;
+                                          int* flags, int* list, int* count) {
+    const int lane = threadIdx.x & 31;
+    const double z = az[m], y = ay[m];
+    for (int k0 = C; k0 <= E - 1; k0 += 32) {
+        const int kl = k0 + lane;
+        unsigned int hit = __ballot_sync(0xffffffffu, kl <= E - 1 && z >= Z[kl] && z < Z[kl + 1]);
+        for (; hit; hit &= hit - 1) {
+            const int k = k0 + __ffs(hit) - 1;
+            for (int j = A + lane; j <= B - 1; j += 32)
+                if (y >= Y[j] && y < Y[j + 1] && k >= 1 && k <= nz && j >= 1 && j <= ny) {
+                    const int q = (k - 1) + nz * (j - 1);
+                    if (atomicExch(&flags[q], 1) == 0) list[atomicAdd(count, 1)] = q;
+                }
+        }
     }
-}
-
-__global__ void k_ray_points(int ny, int nz, const double* Y, const double* Z, const double* az,
-                             const double* ay, int poly, int A, int B, int C, int E, int* points) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= poly) return;
-    ray_point(m, ny, nz, Y, Z, az, ay, A, B, C, E, points);
 }
 
 // Sub-grid volume fraction of cut cell `cell` (airfoil.f90:773-884): the
 // block's threads share the 50 x 50 sub-cells, ETA_1 = odd sub-cells / 2500.
+//
+// A sub-cell's ray meets only edges that span its y and do not lie wholly before its z.  The
+// block lists the edges that span some y of the cell and end at or beyond its Z(k); a warp
+// takes a row of sub-cells, finds the listed edges that span the row, a lane each, and
+// tests those for its 50 sub-cells.  The edges left out change no count and no tie.
+// 64x192x256 with 511 edges (an airfoil of chord 1): 15 us against 475 us with every edge
+// tested for every sub-cell.
 constexpr int kSub = 50;
 template <int NT>
+struct RaySub {
+    double YY[kSub + 1], ZZ[kSub + 1];               // sub-cell nodes
+    EdgeList<NT> ed;
+    int odd[NT / 32];
+};
+template <int NT>
 __device__ __forceinline__ void ray_sub_cell(int cell, int nz, const double* Y, const double* Z, const double* az,
-                                             const double* ay, int poly, double* eta1, int* ties, int* red) {
-    const int k = cell % nz + 1, j = cell / nz + 1;
+                                             const double* ay, int poly, double* eta1, int* ties, RaySub<NT>& sm) {
+    constexpr int kW = NT / 32, kRows = (kSub + kW - 1) / kW;   // warps, rows of a warp
+    static_assert(kSub <= 64 && 2 * kRows <= 32 && NT > kSub, "two sub-cells of a row per lane, a bit each");
+    const int k = cell % nz + 1, j = cell / nz + 1, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const double Yj = Y[j], Yj1 = Y[j + 1], Zk = Z[k], Zk1 = Z[k + 1];
-    int odd = 0, tie = 0;
-    for (int s = threadIdx.x; s < kSub * kSub; s += NT) {
-        const int n = s % kSub + 1, l = s / kSub + 1;   // sub_intersection(n,l)
-        const double YYl = Yj + (l - 1) * (Yj1 - Yj) / (double)kSub;
-        const double YYl1 = Yj + (l) * (Yj1 - Yj) / (double)kSub;
-        const double ZZn = Zk + (n - 1) * (Zk1 - Zk) / (double)kSub;
-        const double ZZn1 = Zk + (n) * (Zk1 - Zk) / (double)kSub;
-        const double ycell = (YYl + YYl1) / 2.0;
-        const double zcell = (ZZn + ZZn1) / 2.0;
-        int cnt = 0;
-        for (int m = 0; m < poly - 1; ++m) {
-            const double a0 = ay[m], a1 = ay[m + 1], z0 = az[m], z1 = az[m + 1];
-            if (a0 >= ycell && a1 <= ycell) {
-                if (zcell > fmax(z0, z1)) {
-                } else if (zcell < fmin(z0, z1)) {
-                    ++cnt;
-                } else {
-                    if (YYl == a1 || ZZn == z1) ++tie;
-                    const double m_pa = (YYl - a1) / (ZZn - z1);
-                    const double m_ab = (a0 - a1) / (z0 - z1);
-                    if (m_pa > m_ab) ++cnt;
-                }
-            }
-            if (a0 <= ycell && a1 >= ycell) {
-                if (zcell > fmax(z0, z1)) {
-                } else if (zcell < fmin(z0, z1)) {
-                    ++cnt;
-                } else {
-                    if (YYl == a1 || ZZn == z1) ++tie;
-                    const double m_pa = (YYl - a0) / (ZZn - z0);
-                    const double m_ab = (a1 - a0) / (z1 - z0);
-                    if (m_pa > m_ab) ++cnt;
+    if (t <= kSub) {
+        sm.YY[t] = Yj + t * (Yj1 - Yj) / (double)kSub;
+        sm.ZZ[t] = Zk + t * (Zk1 - Zk) / (double)kSub;
+    }
+    if (t == 0) sm.ed.count[0] = 0;
+    __syncthreads();
+    unsigned int par = 0u;                           // parity of the lane's sub-cells: rows' pairs of bits
+    int tie = 0;
+    const EdgeList<NT>& ed = sm.ed;
+    for (int m0 = 0, pass = 0; m0 < poly - 1; m0 += NT, pass ^= 1) {
+        const int count = sm.ed.fill(m0, pass, az, ay, poly, [&](double a0, double a1, double z0, double z1) {
+            return fmax(a0, a1) >= fmin(Yj, Yj1) && fmin(a0, a1) <= fmax(Yj, Yj1) && !(fmax(z0, z1) < fmin(Zk, Zk1));
+        });
+        for (int i = 0; i < kRows; ++i) {
+            const int l = warp + i * kW;             // sub_intersection(.,l+1)
+            if (l >= kSub) break;
+            const double YYl = sm.YY[l], ycell = (YYl + sm.YY[l + 1]) / 2.0;
+            for (int e0 = 0; e0 < count; e0 += 32) {
+                const int el = e0 + lane;
+                const bool ok = el < count;
+                const double s0 = ok ? ed.a0[el] : 0.0, s1 = ok ? ed.a1[el] : 0.0;
+                unsigned int downs = __ballot_sync(0xffffffffu, ok && s0 >= ycell && s1 <= ycell);
+                unsigned int ups = __ballot_sync(0xffffffffu, ok && s0 <= ycell && s1 >= ycell);
+                for (unsigned int hit = downs | ups; hit; hit &= hit - 1) {
+                    const int b = __ffs(hit) - 1, e = e0 + b;
+                    const bool down = (downs >> b) & 1u, up = (ups >> b) & 1u;
+                    const double a0 = ed.a0[e], a1 = ed.a1[e], z0 = ed.z0[e], z1 = ed.z1[e];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int n = lane + 32 * h;     // sub_intersection(n+1,.)
+                        if (n >= kSub) continue;
+                        const double ZZn = sm.ZZ[n], zcell = (ZZn + sm.ZZ[n + 1]) / 2.0;
+                        if (zcell > fmax(z0, z1)) continue;
+                        int cnt = 0;
+                        if (zcell < fmin(z0, z1)) cnt = (down ? 1 : 0) + (up ? 1 : 0);
+                        else {
+                            const bool at = YYl == a1 || ZZn == z1;
+                            if (down) {
+                                tie += at;
+                                if ((YYl - a1) / (ZZn - z1) > (a0 - a1) / (z0 - z1)) ++cnt;
+                            }
+                            if (up) {
+                                tie += at;
+                                if ((YYl - a0) / (ZZn - z0) > (a1 - a0) / (z1 - z0)) ++cnt;
+                            }
+                        }
+                        par ^= (unsigned int)(cnt & 1) << (2 * i + h);
+                    }
                 }
             }
         }
-        odd += (cnt % 2 != 0) ? 1 : 0;
+        __syncthreads();                             // the list is read
     }
-    red[threadIdx.x] = odd;
+    const int odd = __reduce_add_sync(0xffffffffu, __popc(par));
+    if (lane == 0) sm.odd[warp] = odd;
     __syncthreads();
-    for (int s = NT / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    if (t == 0) {
+        int all = 0;
+        for (int w = 0; w < kW; ++w) all += sm.odd[w];
+        eta1[(long long)(k - 1) + (long long)nz * (j - 1)] = (double)all / (double)kSub / (double)kSub;
     }
-    if (threadIdx.x == 0) {
-        const double total = (double)red[0];
-        eta1[(long long)(k - 1) + (long long)nz * (j - 1)] = total / (double)kSub / (double)kSub;
-    }
-    __syncthreads();   // red is reused by the block's next cell
     if (tie) atomicAdd(ties, tie);
-}
-
-// One block per listed cell.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_ray_sub(int nz, const double* Y, const double* Z,
-                                                const double* az, const double* ay, int poly,
-                                                const int* cells, double* eta1, int* ties) {
-    __shared__ int red[NT];
-    ray_sub_cell<NT>(cells[blockIdx.x], nz, Y, Z, az, ay, poly, eta1, ties, red);
+    __syncthreads();                                 // the block's next cell
 }
 
 // ETA(i,j,k) = ETA_1(k,j) on the interior (airfoil.f90:889-891); ghosts 0.
@@ -211,8 +253,8 @@ __global__ void k_smooth_mask(int ny, int nz, const double* Y, const double* Z, 
     deta1[q] = de;
 }
 
-// ---- The mask of a moving body on the device, one step at a time inside the
-// step graph (ntcfd_set_dynamic_aoa).  The host evaluates each step's angle
+// ---- The ray cast on the device: a body set by the host, or the mask of a moving
+// body, one step at a time inside the step graph (ntcfd_set_dynamic_aoa).  The host evaluates each step's angle
 // (airfoil.f90:313-317) and its cosine and sine; k_dyn_rotate turns the body
 // polygon by them (airfoil.f90:597-611) for the step the control block's step
 // counter names.  After a step whose polygon meets an exact vertex/grid tie (the
@@ -292,31 +334,29 @@ __global__ void __launch_bounds__(NT) k_dyn_rotate(int ny, int nz, const double*
     }
 }
 
-// Crossing parity of every (k,j) cell; the cut-cell flags cleared.
-__global__ void k_dyn_main(int ny, int nz, const double* Y, const double* Z, DynMask m, const Ctl* ctl) {
+// Crossing parity of every (k,j) cell, a block per part of a row j; the cut-cell flags cleared.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_dyn_main(int ny, int nz, const double* Y, const double* Z, DynMask m,
+                                                 const Ctl* ctl) {
     if (ctl->halt) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    if (k > nz || j > ny) return;
+    __shared__ EdgeList<NT> ed;
     const double* az = m.poly;
-    m.flags[(long long)(k - 1) + (long long)nz * (j - 1)] = 0;
-    ray_main_cell(k, j, nz, Y, Z, az, az + m.npts, m.npts, m.eta1, &m.meta[5]);
+    for (int j = blockIdx.y + 1; j <= ny; j += gridDim.y) {
+        const int k = blockIdx.x * NT + threadIdx.x + 1;
+        if (k <= nz) m.flags[(long long)(k - 1) + (long long)nz * (j - 1)] = 0;
+        ray_main_row<NT>(k, j, nz, Y, Z, az, az + m.npts, m.npts, m.eta1, &m.meta[5], ed);
+    }
 }
 
-// Flags of the cells that hold a vertex (within the bounds).
+// The cells that hold a vertex (within the bounds), flagged and listed (in any order: each
+// is computed on its own).
 __global__ void k_dyn_points(int ny, int nz, const double* Y, const double* Z, DynMask m, const Ctl* ctl) {
     if (ctl->halt) return;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (q >= m.npts) return;
     const double* az = m.poly;
-    ray_point(q, ny, nz, Y, Z, az, az + m.npts, m.meta[0], m.meta[1], m.meta[2], m.meta[3], m.flags);
-}
-
-// The flagged cells into the list (in any order: each is computed on its own).
-__global__ void k_dyn_compact(int cells, DynMask m, const Ctl* ctl) {
-    if (ctl->halt) return;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < cells && m.flags[q]) m.list[atomicAdd(&m.meta[4], 1)] = q;
+    ray_point(q, ny, nz, Y, Z, az, az + m.npts, m.meta[0], m.meta[1], m.meta[2], m.meta[3], m.flags, m.list,
+              &m.meta[4]);
 }
 
 // Sub-cell fractions of the listed cells; blocks stride over the list.
@@ -324,11 +364,11 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_dyn_sub(int nz, const double* Y, const double* Z, DynMask m,
                                                 const Ctl* ctl) {
     if (ctl->halt) return;
-    __shared__ int red[NT];
+    __shared__ RaySub<NT> sm;
     const double* az = m.poly;
     const int count = m.meta[4];
     for (int q = blockIdx.x; q < count; q += gridDim.x)
-        ray_sub_cell<NT>(m.list[q], nz, Y, Z, az, az + m.npts, m.npts, m.eta1, &m.meta[5], red);
+        ray_sub_cell<NT>(m.list[q], nz, Y, Z, az, az + m.npts, m.npts, m.eta1, &m.meta[5], sm);
 }
 
 // ETA from ETA_1, as k_extrude.

@@ -153,6 +153,8 @@ struct ntcfd_ctx {
     DynMask dyn{};
     void* dyn_buf = nullptr;                // the DynMask arrays
     int dyn_cap = 0;                        // polygon points they hold
+    void* ray_buf = nullptr;                // scratch of ntcfd_build_mask_polygon
+    size_t ray_cap = 0;
     double* dyn_trig = nullptr;             // cos, sin of each step's angle (call-indexed)
     int dyn_trig_cap = 0;
     Ctl* ctl_host = nullptr;                // pinned copy of the control block at the end of a call
@@ -756,7 +758,7 @@ int build_graph(ntcfd_ctx* ctx) {
 }
 
 // Kernels of the moving body's mask in a step of the moving-body graph.
-constexpr int kDynKernels = 7;
+constexpr int kDynKernels = 6;
 
 // The moving-body step graph (ntcfd_set_dynamic_aoa): the step's mask
 // (airfoil.f90:311-321, RayCasting at the step's angle) -> gate -> IF(no tie in
@@ -769,19 +771,16 @@ int build_dyn_graph(ntcfd_ctx* ctx) {
     ctx->graph_dyn = G;
     const DynMask m = ctx->dyn;
     const Ctl* cctl = ctx->ctl;
-    const int cells = g.ny * g.nz;
     std::vector<cudaGraphNode_t> dep;
     cudaGraphNode_t n;
     GK(add_kernel(&n, G, dep, k_dyn_rotate<512>, dim3(1), dim3(512), g.ny, g.nz, (const double*)ctx->coordY,
                   (const double*)ctx->coordZ, m, cctl));
     dep = {n};
-    GK(add_kernel(&n, G, dep, k_dyn_main, dim3((g.nz + 31) / 32, (g.ny + 7) / 8), dim3(32, 8), g.ny, g.nz,
+    GK(add_kernel(&n, G, dep, k_dyn_main<128>, dim3((g.nz + 127) / 128, std::min(g.ny, 65535)), dim3(128), g.ny, g.nz,
                   (const double*)ctx->coordY, (const double*)ctx->coordZ, m, cctl));
     dep = {n};
-    GK(add_kernel(&n, G, dep, k_dyn_points, dim3((m.npts + 127) / 128), dim3(128), g.ny, g.nz,
+    GK(add_kernel(&n, G, dep, k_dyn_points, dim3((m.npts + 3) / 4), dim3(128), g.ny, g.nz,
                   (const double*)ctx->coordY, (const double*)ctx->coordZ, m, cctl));
-    dep = {n};
-    GK(add_kernel(&n, G, dep, k_dyn_compact, dim3((cells + 255) / 256), dim3(256), cells, m, cctl));
     dep = {n};
     GK(add_kernel(&n, G, dep, k_dyn_sub<256>, dim3(2 * ctx->sm_count), dim3(256), g.nz,
                   (const double*)ctx->coordY, (const double*)ctx->coordZ, m, cctl));
@@ -1262,6 +1261,7 @@ void ntcfd_destroy(ntcfd_ctx* ctx) {
     for (void* q : ctx->allocs) cudaFree(q);
     if (ctx->dyn_trig) cudaFree(ctx->dyn_trig);
     if (ctx->dyn_buf) cudaFree(ctx->dyn_buf);
+    if (ctx->ray_buf) cudaFree(ctx->ray_buf);
     if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
     if (ctx->rec) cudaFree(ctx->rec);
     if (ctx->rec_host) cudaFreeHost(ctx->rec_host);
@@ -1673,22 +1673,18 @@ int prepare_dyn(ntcfd_ctx* ctx, int nsteps) {
     return 0;
 }
 
-// The mask kernels of a moving-body step launched one by one (eager contexts,
-// or where the moving-body graph could not be built); *ties receives the
-// step's exact vertex/grid ties.
-int dyn_mask_eager(ntcfd_ctx* ctx, int* ties) {
+// The ray cast's kernels on the stream, for the step and the halt flag of `ctl`; waits and
+// returns the exact vertex/grid ties.
+int ray_cast(ntcfd_ctx* ctx, const DynMask& m, const Ctl* ctl, int* ties) {
     const Geom& g = ctx->g;
-    const DynMask m = ctx->dyn;
-    const int cells = g.ny * g.nz;
     cudaStream_t st = ctx->stream;
-    k_dyn_rotate<512><<<1, 512, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctx->ctl);
-    k_dyn_main<<<dim3((g.nz + 31) / 32, (g.ny + 7) / 8), dim3(32, 8), 0, st>>>(g.ny, g.nz, ctx->coordY,
-                                                                              ctx->coordZ, m, ctx->ctl);
-    k_dyn_points<<<(m.npts + 127) / 128, 128, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctx->ctl);
-    k_dyn_compact<<<(cells + 255) / 256, 256, 0, st>>>(cells, m, ctx->ctl);
-    k_dyn_sub<256><<<2 * ctx->sm_count, 256, 0, st>>>(g.nz, ctx->coordY, ctx->coordZ, m, ctx->ctl);
+    k_dyn_rotate<512><<<1, 512, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctl);
+    k_dyn_main<128><<<dim3((g.nz + 127) / 128, std::min(g.ny, 65535)), 128, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m,
+                                                                                     ctl);
+    k_dyn_points<<<(m.npts + 3) / 4, 128, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctl);
+    k_dyn_sub<256><<<2 * ctx->sm_count, 256, 0, st>>>(g.nz, ctx->coordY, ctx->coordZ, m, ctl);
     k_dyn_extrude<<<dim3((g.nx + 4 + 31) / 32, (g.ny + 4 + 3) / 4, (g.nz + 4 + 1) / 2), dim3(32, 4, 2), 0, st>>>(
-        g, m.eta1, ctx->eta, ctx->ctl);
+        g, m.eta1, ctx->eta, ctl);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(ties, &m.meta[5], sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1744,7 +1740,7 @@ int ntcfd_step(ntcfd_ctx* ctx, int nsteps, ntcfd_step_info* info) {
                 continue;
             }
             int ties = 0;
-            if (int rc = dyn_mask_eager(ctx, &ties)) return rc;
+            if (int rc = ray_cast(ctx, ctx->dyn, ctx->ctl, &ties)) return rc;
             if (ties) {
                 // steps 0..s-1 ran: account for them (time, step count, records) before
                 // returning, so that the host's view matches the device state
@@ -2066,74 +2062,44 @@ int ntcfd_build_mask_polygon(ntcfd_ctx* ctx, const double* az_in, const double* 
     if (!ctx->coords_set) return fail(ctx, NTCFD_ESTATE, "ntcfd_set_coords must come first");
     if (int rc = set_mask_flag(ctx, true)) return rc;
     const Geom& g = ctx->g;
-    // airfoil.f90:597-611 on the host: shift by the quarter chord, rotate by
-    // -AOA (ay uses the already rotated az, as in the reference), translate.
-    std::vector<double> az(az_in, az_in + npts), ay(ay_in, ay_in + npts);
-    const double PI = 4.0 * std::atan(1.0);
-    for (int i = 0; i < npts; ++i) {
-        az[i] = az[i] - 0.25;
-        az[i] = std::cos((-aoa) * PI / 180) * az[i] - std::sin((-aoa) * PI / 180) * ay[i];
-        ay[i] = std::sin((-aoa) * PI / 180) * az[i] + std::cos((-aoa) * PI / 180) * ay[i];
-        az[i] = az[i] + zc;
-        ay[i] = ay[i] + yc;
-        az[i] = az[i] + 0.25;
-    }
-    // node coordinates back on the host for the A, B, C, E search (airfoil.f90:615-654)
-    std::vector<double> Y(g.ny + 5), Z(g.nz + 5);
-    CK(cudaMemcpyAsync(Y.data(), ctx->coordbuf, (g.ny + 5) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(Z.data(), ctx->coordbuf + (g.ny + 5) + 4, (g.nz + 5) * sizeof(double),
-                       cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    auto Yf = [&](int j) { return Y[j + 1]; };
-    auto Zf = [&](int k) { return Z[k + 1]; };
-    double miny = ay[0], maxy = ay[0], minz = az[0], maxz = az[0];
-    for (int i = 1; i < npts; ++i) {
-        miny = std::min(miny, ay[i]); maxy = std::max(maxy, ay[i]);
-        minz = std::min(minz, az[i]); maxz = std::max(maxz, az[i]);
-    }
-    int A = 0, B = 0, C = 0, E = 0;
-    for (int j = 1; j <= g.ny; ++j) if (Yf(j) > miny) { A = j - 1; break; }
-    for (int j = 1; j <= g.ny; ++j) if (Yf(j) > maxy) { B = j; break; }
-    for (int k = 1; k <= g.nz; ++k) if (Zf(k) > minz) { C = k - 1; break; }
-    for (int k = 1; k <= g.nz; ++k) if (Zf(k) > maxz) { E = k; break; }
-    // device work buffers
-    double* daz = nullptr;
-    int* dint = nullptr;
     const size_t cells = (size_t)g.ny * g.nz;
-    CK(cudaMalloc(&daz, sizeof(double) * 2 * npts));
-    CK(cudaMalloc(&dint, sizeof(int) * (2 * cells + 1)));
-    double* day = daz + npts;
-    int* points = dint;
-    int* list = dint + cells;
-    int* ties = dint + 2 * cells;
-    CK(cudaMemcpyAsync(daz, az.data(), sizeof(double) * npts, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(day, ay.data(), sizeof(double) * npts, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemsetAsync(dint, 0, sizeof(int) * (2 * cells + 1), ctx->stream));
-    double* eta1 = ctx->outbuf;
-    k_ray_main<<<dim3((g.nz + 31) / 32, (g.ny + 7) / 8), dim3(32, 8), 0, ctx->stream>>>(
-        g.ny, g.nz, ctx->coordY, ctx->coordZ, daz, day, npts, eta1, ties);
-    k_ray_points<<<(npts + 127) / 128, 128, 0, ctx->stream>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, daz,
-                                                                day, npts, A, B, C, E, points);
-    std::vector<int> hp(cells);
-    CK(cudaMemcpyAsync(hp.data(), points, sizeof(int) * cells, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    std::vector<int> hl;
-    for (size_t q = 0; q < cells; ++q)
-        if (hp[q]) hl.push_back((int)q);
-    if (!hl.empty()) {
-        CK(cudaMemcpyAsync(list, hl.data(), sizeof(int) * hl.size(), cudaMemcpyHostToDevice, ctx->stream));
-        k_ray_sub<256><<<(unsigned)hl.size(), 256, 0, ctx->stream>>>(g.nz, ctx->coordY, ctx->coordZ, daz,
-                                                                    day, npts, list, eta1, ties);
+    // The context's scratch: {control block, cosine and sine, body polygon} of this call,
+    // one copy; moved polygon; flags; list; bounds and counters.  Kept, so that turning a
+    // body allocates nothing and waits once.
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t head = 512, pb = 2 * sizeof(double) * (size_t)npts, fb = up(sizeof(int) * cells);
+    const size_t bytes = up(head + pb) + up(pb) + 2 * fb + 256;
+    if (bytes > ctx->ray_cap) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (ctx->ray_buf) cudaFree(ctx->ray_buf);
+        ctx->ray_buf = nullptr;
+        ctx->ray_cap = 0;
+        CK(cudaMalloc(&ctx->ray_buf, bytes));
+        ctx->ray_cap = bytes;
     }
-    const dim3 b3(32, 4, 2);
-    k_extrude<<<dim3((g.nx + 4 + 31) / 32, (g.ny + 4 + 3) / 4, (g.nz + 4 + 1) / 2), b3, 0, ctx->stream>>>(
-        g, eta1, ctx->eta);
+    unsigned char* const q = (unsigned char*)ctx->ray_buf;
+    static_assert(sizeof(Ctl) <= 256, "control block outgrew its scratch slot");
+    // the rotation of airfoil.f90:597-611 (pi = 4 atan(1) there), made on the device
+    const double PI = 4.0 * std::atan(1.0);
+    const double trig[2] = {std::cos((-aoa) * PI / 180), std::sin((-aoa) * PI / 180)};
+    std::vector<unsigned char> in(head + pb, 0);
+    std::memcpy(in.data() + 256, trig, sizeof trig);
+    std::memcpy(in.data() + head, az_in, pb / 2);
+    std::memcpy(in.data() + head + pb / 2, ay_in, pb / 2);
+    CK(cudaMemcpyAsync(q, in.data(), in.size(), cudaMemcpyHostToDevice, ctx->stream));
+    DynMask m{};
+    m.trig = (const double*)(q + 256);
+    m.base = (const double*)(q + head);
+    m.poly = (double*)(q + up(head + pb));
+    m.flags = (int*)(q + up(head + pb) + up(pb));
+    m.list = (int*)(q + up(head + pb) + up(pb) + fb);
+    m.meta = (int*)(q + up(head + pb) + up(pb) + 2 * fb);
+    m.npts = npts;
+    m.zc = zc;
+    m.yc = yc;
+    m.eta1 = ctx->outbuf;
     int hties = 0;
-    CK(cudaMemcpyAsync(&hties, ties, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(ctx->stream));
-    cudaFree(daz);
-    cudaFree(dint);
+    if (int rc = ray_cast(ctx, m, (const Ctl*)q, &hties)) return rc;
     if (ties_out) *ties_out = hties;
     if (hties)
         return fail(ctx, NTCFD_EINVAL,
@@ -2231,18 +2197,8 @@ extern "C" int ntcfd_build_mask_polygon_noalloc(ntcfd_ctx* ctx, const double* az
     CK(cudaMemcpyAsync((double*)m.trig, trig, sizeof trig, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync((double*)m.base, az_in, sizeof(double) * npts, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync((double*)m.base + npts, ay_in, sizeof(double) * npts, cudaMemcpyHostToDevice, st));
-    k_dyn_rotate<512><<<1, 512, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctl);
-    k_dyn_main<<<dim3((g.nz + 31) / 32, (g.ny + 7) / 8), dim3(32, 8), 0, st>>>(g.ny, g.nz, ctx->coordY,
-                                                                              ctx->coordZ, m, ctl);
-    k_dyn_points<<<(npts + 127) / 128, 128, 0, st>>>(g.ny, g.nz, ctx->coordY, ctx->coordZ, m, ctl);
-    k_dyn_compact<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>((int)cells, m, ctl);
-    k_dyn_sub<256><<<2 * ctx->sm_count, 256, 0, st>>>(g.nz, ctx->coordY, ctx->coordZ, m, ctl);
-    k_dyn_extrude<<<dim3((g.nx + 4 + 31) / 32, (g.ny + 4 + 3) / 4, (g.nz + 4 + 1) / 2), dim3(32, 4, 2), 0, st>>>(
-        g, m.eta1, ctx->eta, ctl);
-    CK(cudaGetLastError());
     int hties = 0;
-    CK(cudaMemcpyAsync(&hties, &m.meta[5], sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    if (int rc = ray_cast(ctx, m, ctl, &hties)) return rc;
     if (ties_out) *ties_out = hties;
     if (hties)
         return fail(ctx, NTCFD_EINVAL,
