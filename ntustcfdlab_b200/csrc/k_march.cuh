@@ -249,9 +249,7 @@ __device__ __forceinline__ Rows<double> fma_rn(Rows<double> a, Rows<double> b, R
 __device__ __forceinline__ Rows<double> add_rn(Rows<double> a, Rows<double> b) { return {a.v + b.v}; }
 __device__ __forceinline__ Rows<double> sub_rn(Rows<double> a, Rows<double> b) { return {sub_rn(a.v, b.v)}; }
 
-// 1 / diag of the coefficient sum s, with the coefficients' sign.  FP32: to nearest for
-// a normal sum with a normal reciprocal, the hardware's approximation and one
-// Newton-Raphson step, whose remainder the FMA keeps exactly.
+// 1 / diag of the coefficient sum s, with the coefficients' sign (rdiag32, two rows at once).
 __device__ __forceinline__ Rows<float> march_rd(Rows<float> s) {
     float a, b;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(-s.get(0)));

@@ -76,6 +76,16 @@ __device__ __forceinline__ double rdiag64(double s) {
     return x;
 }
 
+// FP32, to nearest for a normal sum with a normal reciprocal: the hardware's approximation
+// and one Newton-Raphson step, whose remainder the FMA keeps exactly.
+__device__ __forceinline__ float rdiag32(float s) {
+    float x;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(s));
+    return fma_rn(x, fma_rn(-s, x, 1.0f), x);
+}
+__device__ __forceinline__ float rdiag_near(float s) { return rdiag32(s); }
+__device__ __forceinline__ double rdiag_near(double s) { return rdiag64(s); }
+
 // The FP64 defect of p + e from the defect d of p and the correction e of a
 // defect-correction cycle: since the operator is linear,
 //     d' = rdiag sum c (p+e)_nb - b' - (p+e) = d + rdiag sum_nb c_nb e_nb - e,
