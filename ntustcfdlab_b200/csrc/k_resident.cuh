@@ -649,6 +649,11 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
                 if ((int)((unsigned int)wr - target) < 0 &&
                     !count_wait(&sync->cnt[0][sg & 3], target, &sync->bar.err, &wr))
                     s_fail[par] = 1;
+                // every verdict of that half counts: a late one would be taken for the next use of its counter
+                const unsigned int before = nblocks * (unsigned)(((sg + 3) >> 2));
+                if ((int)((unsigned int)wb - before) < 0 &&
+                    !count_wait(&sync->cnt[1][(sg + 3) & 3], before, &sync->bar.err, &wb))
+                    s_fail[par] = 1;
                 const unsigned int h0 = (unsigned int)(wr >> 32), h1 = (unsigned int)(wb >> 32);
                 s_vd = make_uint2(h0 - s_prev[0][sg & 3], sg > 0 ? h1 - s_prev[1][(sg + 3) & 3] : 0u);
                 s_prev[0][sg & 3] = h0;
