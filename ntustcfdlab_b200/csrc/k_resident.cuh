@@ -68,6 +68,7 @@ struct Brick {
     int cache_rd;    // 1: rd of the brick lives in shared memory too
     int mode;        // kResNarrow, kResWide1 or kResWide (res_mode(nx))
     int inbox;       // ring words per CTA and colour
+    int deep;        // 1: k_sor_deep (k_resident_deep.cuh)
 };
 
 // Cells of a colour in a row: (nx + r) / 2 for parity r; at most (nx + 1) / 2.

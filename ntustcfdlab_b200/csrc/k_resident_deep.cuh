@@ -13,13 +13,20 @@
 // read a sweep's words when the next sweep's arrive, but has read them before the
 // ones after (it published those of the sweep between, which this CTA waited for).
 //
-// The stop rule is the resident kernel's: the red halves' verdicts decide unless no red cell
-// changed by more than zeta; here they travel while the black words do.  Restarts
+// The stop rule (k_resident.cuh).  The verdicts of a sweep's two halves take longer to
+// be summed over the CTAs than a sweep, so they are judged one sweep later: a solve that
+// turns out to have ended a sweep ago takes e from before this sweep, which every update
+// leaves beside the new value.  A cycle's last sweep is judged at once.  Restarts
 // and the final p += e run in the kernel; d of the first ring row's red cells is kept
 // and updated like the brick's own.  1/diag is formed from the coefficients.
 // Rows of at most 32 cells per colour, two or more side by side on a warp's lanes.
 //
-// Measured: DEEP_FIGURES
+// A sweep takes 2.6 us at 40^3 FP64 (3.3 with two hand-overs), 2.6 us at 61x47x53 FP32 (3.5),
+// 2.7 us at 32x96x96 FP32 (3.8), 1.6 us at 12x10x8 FP64 (2.3, in one CTA).  Bound by the
+// hand-over's trip (1.5 us) and, past some 40 rows a brick, by instruction issue: a turn of the 16
+// warps over a row each takes 0.28 us FP32, 0.35 us FP64.  One row per warp and turn: with two, as
+// the resident kernel takes them, half of a small brick's last turn is empty (32x96x96: 2.95 us).
+// The verdicts judged in their own sweep: 3.0 us there.
 #pragma once
 
 #include "k_resident.cuh"
@@ -34,10 +41,10 @@ __host__ __device__ inline int deep_inbox_rows(const Brick& b) { return 4 * (b.J
 
 template <class Tc>
 inline size_t deep_smem(const Brick& b) {
-    // e and d of both colours, 64 words of slack (loads past the last row), then per red row its
+    // e, d and the sweep before's e of both colours, 64 words of slack (loads past the last row), then per red row its
     // coefficients and place, per own row its places in up to eight inboxes, the ring list
-    return sizeof(Tc) * (4 * (size_t)deep_tile_rows(b) * b.mx + 64) + (size_t)deep_red_rows(b) * (4 * sizeof(Tc) + 8) +
-           (size_t)b.JB * b.KB * 32 + (size_t)deep_inbox_rows(b) * 12 + 32;
+    return sizeof(Tc) * (6 * (size_t)deep_tile_rows(b) * b.mx + 64) + (size_t)deep_red_rows(b) * (4 * sizeof(Tc) + 8) +
+           (size_t)b.JB * b.KB * 32 + (size_t)deep_inbox_rows(b) * 12 + 64;
 }
 
 template <class Tc, int NT>
@@ -61,9 +68,12 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     Tc* const D1 = D0 + tile;
     // per red row (own rows first): cN, cS, cF, cB; tile row start and (j+k)&1
     const int nrmax = deep_red_rows(br);
-    Tc* const rowC = D1 + tile + 64;
+    Tc* const H0 = D1 + tile;                     // own cells' e before the last sweep
+    Tc* const H1 = H0 + tile;
+    auto align16 = [&](const void* q) { return smem_raw + (((size_t)((const unsigned char*)q - smem_raw) + 15) & ~size_t(15)); };
+    Tc* const rowC = reinterpret_cast<Tc*>(align16(H1 + tile + 64));
     int2* const rowT = reinterpret_cast<int2*>(rowC + 4 * nrmax);
-    int* const pubT = reinterpret_cast<int*>(rowT + nrmax);      // eight per own row, -1: no more
+    int* const pubT = reinterpret_cast<int*>(align16(rowT + nrmax));      // words into the inboxes, eight per own row, -1: none
     int* const ringT = pubT + 8 * JB * KB;                       // inbox row, tile row start, (j+k)&1
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -74,7 +84,7 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     const int nown0 = g.nx / 2, nown1 = (g.nx + 1) / 2, nrows = nj * nk;
     auto place = [&](int jl, int kl) { return ((kl + 1) * RS + jl + 1) * mx; };   // jl, kl = -1 .. n + 2
 
-    for (int q = tid; q < 4 * tile + 64; q += NT) S0[q] = Tc(0);
+    for (int q = tid; q < 6 * tile + 64; q += NT) S0[q] = Tc(0);
     if (tid == 0) {
         s_fail[0] = s_fail[1] = s_nan[0] = s_nan[1] = 0;
         s_vd = make_uint2(0u, 0u);
@@ -97,9 +107,9 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
         const int jl = er % nj + 1, kl = er / nj + 1;
         red_row(er, jl, kl);
         int n = 0;
-        // the neighbour one brick along (dj, dk) keeps this row at `row` of its inbox
+        // the neighbour one brick along (dj, dk) keeps this row at `row` of its inbox (the first half's)
         auto to = [&](int dj, int dk, int row) {
-            pubT[8 * er + n++] = ((int)blockIdx.x + dj + dk * br.nbj) * 2 * rows_in + row;
+            pubT[8 * er + n++] = (((int)blockIdx.x + dj + dk * br.nbj) * 2 * rows_in + row) * nown1 * Word::n;
         };
         if (jlo && jl <= 2) to(-1, 0, 2 * KB + (jl - 1) * KB + kl - 1);                  // its j-high face
         if (jhi && jl >= nj - 1) to(1, 0, (nj - jl) * KB + kl - 1);                      // its j-low face
@@ -110,7 +120,7 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
         if (jhi && klo && jl == nj && kl == 1) to(1, -1, corner + 2);
         if (jlo && khi && jl == 1 && kl == nk) to(-1, 1, corner + 1);
         if (jhi && khi && jl == nj && kl == nk) to(1, 1, corner + 0);
-        if (n < 8) pubT[8 * er + n] = -1;
+        while (n < 8) pubT[8 * er + n++] = -1;
     }
     // the first ring row's red rows, and the rows that come from the inbox (black), in any order
     for (int q = tid; q < rows_in; q += NT) {
@@ -170,54 +180,51 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     const unsigned int mH = 0xffffffffu / (unsigned)nown1 + 1u;  // q / nown1
     __syncthreads();
 
-    // one colour over the first n rows; black is published under seq
+    // one colour over the first n rows, rpw rows per warp and turn; black is published under seq
     auto pass = [&](auto cc, int n, unsigned int seq, B& ch) {
         constexpr int c = decltype(cc)::value;
         Tc* const W = c ? S1 : S0;
         const Tc* const O = c ? S0 : S1;
         const Tc* const D = c ? D1 : D0;
-        unsigned long long* const box = boxes + (seq & 1u) * boxw;
-        for (int er = 2 * rpw * warp + sub; er < n + sub; er += 2 * rpw * NWARP) {
-            Tc e1[2], diff[2];
-            int m[2], row[2];
-            bool ok[2], in[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int e = er + h * rpw;
-                in[h] = sub < rpw && e < n;
-                row[h] = in[h] ? e : 0;
-                const int2 rt = rowT[row[h]];
-                const int r = (rt.y ^ c) & 1;
-                m[h] = rt.x + lt + 2 - r;
-                ok[h] = in[h] && lt < (r ? nown1 : nown0);
-                const Tc* const o = O + m[h];
-                const Tc* const rc = rowC + 4 * row[h];
-                const Tc cN = rc[0], cS = rc[1], cF = rc[2], cB = rc[3];
-                const Tc cE = r ? cEr[1] : cEr[0], cW = r ? cWr[1] : cWr[0];
-                const Tc rd = rdiag_near(((cE + cW) + (cN + cS)) + (cF + cB));
-                diff[h] = sor_update(cE, O[rt.x + lt + 2], cW, O[rt.x + lt + 1], cN, o[mx], cS, o[-mx], cF, o[plane], cB,
-                                     o[-plane], rd, D[m[h]], W[m[h]], om, &e1[h]);
+        Tc* const H = c ? H1 : H0;
+        unsigned long long* const box = boxes + (seq & 1u) * boxw + lt * Word::n;
+        for (int er = rpw * warp + sub; er < n + sub; er += rpw * NWARP) {
+            const bool in = sub < rpw && er < n;
+            const int row = in ? er : 0;
+            const int2 rt = rowT[row];
+            const int r = (rt.y ^ c) & 1, m = rt.x + lt + 2 - r;
+            const bool ok = in && lt < (r ? nown1 : nown0);
+            const Tc* const o = O + m;
+            Tc cN, cS, cF, cB;
+            if constexpr (sizeof(Tc) == 4) {
+                const float4 q = *reinterpret_cast<const float4*>(rowC + 4 * row);
+                cN = q.x; cS = q.y; cF = q.z; cB = q.w;
+            } else {
+                const double2 q = *reinterpret_cast<const double2*>(rowC + 4 * row);
+                const double2 t = *reinterpret_cast<const double2*>(rowC + 4 * row + 2);
+                cN = q.x; cS = q.y; cF = t.x; cB = t.y;
             }
+            const Tc cE = r ? cEr[1] : cEr[0], cW = r ? cWr[1] : cWr[0], e0 = W[m];
+            const Tc rd = rdiag_near(((cE + cW) + (cN + cS)) + (cF + cB));
+            Tc e1;
+            const Tc diff = sor_update(cE, O[rt.x + lt + 2], cW, O[rt.x + lt + 1], cN, o[mx], cS, o[-mx], cF, o[plane], cB,
+                                       o[-plane], rd, D[m], e0, om, &e1);
+            if (ok) {
+                W[m] = e1;
+                H[m] = e0;
+                if (c || row < nrows) {
+                    const B b = abs_bits(diff);
+                    ch = b > ch ? b : ch;
+                }
+            }
+            if (c && in) {
+                const Tc v = ok ? e1 : Tc(0);     // 0 where the row is a cell shorter than the ring
+                const int4 ta = *reinterpret_cast<const int4*>(pubT + 8 * row);
+                const int4 tb = *reinterpret_cast<const int4*>(pubT + 8 * row + 4);
+                const int to[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (ok[h]) {
-                    W[m[h]] = e1[h];
-                    if (row[h] < nrows) {
-                        const B b = abs_bits(diff[h]);
-                        ch = b > ch ? b : ch;
-                    }
-                }
-                if (c && in[h]) {
-                    const Tc v = ok[h] ? e1[h] : Tc(0);   // 0 where the row is a cell shorter than the ring
-                    const int* const to = pubT + 8 * row[h];
-#pragma unroll 1
-                    for (int q = 0; q < 8; ++q) {
-                        const int t = to[q];
-                        if (t < 0) break;
-                        // inbox row t: of CTA t / (2 rows_in), whose halves are boxw apart
-                        Word::store(box + ((size_t)t * nown1 + lt) * Word::n, v, seq);
-                    }
-                }
+                for (int q = 0; q < 8; ++q)
+                    if (to[q] >= 0) Word::store(box + to[q], v, seq);
             }
         }
     };
@@ -260,7 +267,8 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     };
     // p += e of the own rows, a warp per row; with `defect` also d = the FP64 defect of
     // p + e (defect_update) of every cell whose d is kept
-    auto correct = [&](bool defect) {
+    // (undo: from e before the last sweep)
+    auto correct = [&](bool defect, bool undo) {
         for (int q = warp; q < (defect ? nr : nrows); q += NWARP) {
             const int2 rt = rowT[q];
             const int kl = rt.x / plane - 1, jl = rt.x / mx % RS - 1, j = j0 + jl - 1, k = k0 + kl - 1;
@@ -271,7 +279,7 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
                 if (c && !own) continue;
                 const int r = (rt.y ^ c) & 1, m = rt.x + lane + 2 - r, i = 2 * lane + 2 - r;
                 if (lane >= (r ? nown1 : nown0)) continue;
-                const Tc e = (c ? S1 : S0)[m];
+                const Tc e = undo ? (c ? H1 : H0)[m] : (c ? S1 : S0)[m];
                 double* const pp = p + nat(g, i, j, k);
                 const double pv = own ? *pp : 0.0;
                 if (defect) {
@@ -294,39 +302,44 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     };
     constexpr B kInf = sizeof(Tc) == 4 ? (B)0x7f800000u : (B)kInfBits;
 
+    // The sums of sweep sg's verdicts to s_vd (red, black), once per sweep and in order; by
+    // ctrl, from the counters as it saw them earlier (w).
+    auto look = [&](int sg) {
+        return make_ulonglong2(ld_relaxed(&sync->cnt[0][sg & 3]), ld_relaxed(&sync->cnt[1][sg & 3]));
+    };
+    auto judge = [&](int sg, int par, ulonglong2 w) {
+        const unsigned int target = nblocks * (unsigned)((sg >> 2) + 1);
+        const bool ok = ((int)((unsigned int)w.x - target) >= 0 ||
+                         count_wait(&sync->cnt[0][sg & 3], target, &sync->bar.err, &w.x)) &&
+                        ((int)((unsigned int)w.y - target) >= 0 ||
+                         count_wait(&sync->cnt[1][sg & 3], target, &sync->bar.err, &w.y));
+        if (!ok) s_fail[par] = 1;
+        const unsigned int h0 = (unsigned int)(w.x >> 32), h1 = (unsigned int)(w.y >> 32);
+        s_vd = make_uint2(h0 - s_prev[0][sg & 3], h1 - s_prev[1][sg & 3]);
+        s_prev[0][sg & 3] = h0;
+        s_prev[1][sg & 3] = h1;
+    };
     int done = 0, done_c = 0, restarts = 0;
-    bool conv = false, nonfinite = false, failed = false, tested = false, prev_tested = false;
+    bool conv = false, nonfinite = false, failed = false, tested = false, undo = false, added = false;
     B chs = B(0);
     double last = 0.0;
     for (;;) {
         done_c = 0;
+        bool open = false, open_test = false;         // the sweep before is not judged yet; and is tested
 #pragma unroll 1
         for (int s = 0; ik0 + done + s < itmax && s < cycle_len; ++s) {
             const int sg = done + s, par = sg & 1, ik = ik0 + sg + 1;
-            const unsigned int target = nblocks * (unsigned)((sg >> 2) + 1), seq = seq0 + (unsigned)sg + 1u;
-            const bool test = check_every == 1 || ik >= itmax || ik % check_every == 0;
+            const unsigned int seq = seq0 + (unsigned)sg + 1u;
             B cr = B(0), cb = B(0);
             pass(RedT{}, nr, seq, cr);
             if (cr >= kInf) s_nan[par] = 1;
             const int any_r = __syncthreads_or(above(cr));
             if (ctrl) red_add_relaxed(&sync->cnt[0][sg & 3], verdict(any_r, par));
             pass(BlackT{}, nrows, seq, cb);
-            // the counters' first look: this sweep's red verdicts, the last sweep's black ones
-            unsigned long long wr = 0ull, wb = 0ull;
-            if (ctrl) {
-                wr = ld_relaxed(&sync->cnt[0][sg & 3]);
-                wb = ld_relaxed(&sync->cnt[1][(sg + 3) & 3]);
-            }
+            ulonglong2 w = make_ulonglong2(0ull, 0ull);
+            if (ctrl && open) w = look(sg - 1);       // a trip through L2 ahead of its use
             fill(seq, par);
-            if (ctrl) {
-                if ((int)((unsigned int)wr - target) < 0 &&
-                    !count_wait(&sync->cnt[0][sg & 3], target, &sync->bar.err, &wr))
-                    s_fail[par] = 1;
-                const unsigned int h0 = (unsigned int)(wr >> 32), h1 = (unsigned int)(wb >> 32);
-                s_vd = make_uint2(h0 - s_prev[0][sg & 3], sg > 0 ? h1 - s_prev[1][(sg + 3) & 3] : 0u);
-                s_prev[0][sg & 3] = h0;
-                if (sg > 0) s_prev[1][(sg + 3) & 3] = h1;
-            }
+            if (ctrl && open) judge(sg - 1, par, w);
             if (cb >= kInf) s_nan[par] = 1;
             const int any_b = __syncthreads_or(above(cb));
             if (s_fail[par]) {
@@ -334,46 +347,49 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
                 break;
             }
             if (ctrl) red_add_relaxed(&sync->cnt[1][sg & 3], verdict(any_b, par));
-            const uint2 vd = s_vd;
-            if (prev_tested && vd.y >= kNanFlag) {
-                nonfinite = true;                 // met in the sweep before
-                break;
+            if (open_test) {
+                const uint2 vd = s_vd;
+                nonfinite = vd.x >= kNanFlag || vd.y >= kNanFlag;
+                conv = vd.x == 0u && vd.y == 0u;
+                if (conv || nonfinite) {              // the solve ended with the sweep before
+                    undo = true;
+                    break;
+                }
             }
             chs = cb > cr ? cb : cr;
             done_c = s + 1;
-            prev_tested = test;
-            if (test) {
-                tested = true;
-                unsigned int vb = 1u;
-                if (vd.x < kNanFlag && (vd.x == 0u || ik >= itmax)) {
-                    __syncthreads();              // s_vd has been read
-                    if (ctrl) {
-                        unsigned long long w = 0ull;
-                        if (!count_wait(&sync->cnt[1][sg & 3], target, &sync->bar.err, &w)) s_fail[par] = 1;
-                        s_vd.y = (unsigned int)(w >> 32) - s_prev[1][sg & 3];
-                    }
-                    __syncthreads();
-                    if (s_fail[par]) {
-                        failed = true;
-                        break;
-                    }
-                    vb = s_vd.y;
-                }
-                nonfinite = vd.x >= kNanFlag || vb >= kNanFlag;
-                conv = vd.x == 0u && vb == 0u;
-                if (conv || nonfinite) break;
-            }
+            open = true;
+            open_test = check_every == 1 || ik >= itmax || ik % check_every == 0;
+            tested = tested || open_test;
         }
         done += done_c;
-        // another cycle only when this one ended on its length
-        if (failed || conv || nonfinite || done_c < cycle_len || ik0 + done >= itmax) break;
-        correct(true);
-        __syncthreads();
+        if (failed || undo) break;
+        // another cycle only when this one ended on its length; its p += e and d do no harm to a
+        // solve that turns out to have ended, and cover the judgement
+        const bool again = done_c == cycle_len && ik0 + done < itmax;
+        if (again) correct(true, false);
+        added = again;
+        if (open) {
+            const int par = (done - 1) & 1;
+            __syncthreads();                          // s_vd and s_fail have been read
+            if (ctrl) judge(done - 1, par, look(done - 1));
+            __syncthreads();
+            if (s_fail[par]) {
+                failed = true;
+                break;
+            }
+            if (open_test) {
+                nonfinite = s_vd.x >= kNanFlag || s_vd.y >= kNanFlag;
+                conv = s_vd.x == 0u && s_vd.y == 0u;
+            }
+        }
+        if (conv || nonfinite || !again) break;
+        added = false;
         for (int q = tid; q < 2 * tile; q += NT) S0[q] = Tc(0);
         __syncthreads();
         ++restarts;
     }
-    correct(false);
+    if (!added) correct(false, undo);
     // the max |change| of the last (tested) sweep
     if (!failed && tested && done > 0) {
 #pragma unroll
@@ -393,7 +409,7 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
         else if (tid == 0) last = __longlong_as_double((long long)ld_relaxed(&sync->last));
     }
     if (blockIdx.x == 0 && tid == 0) {
-        sync->seq = seq0 + (failed ? 1u << 24 : (unsigned)done + 4u);
+        sync->seq = seq0 + (failed ? 1u << 24 : (unsigned)done + 8u);
         ctl->ik = ik0 + done;
         ctl->inner = done_c;
         ctl->cycles += restarts + (itmax > 0 ? 1 : 0);   // the launch's cycles, the last included

@@ -30,6 +30,7 @@
 #include "k_pressure.cuh"
 #include "k_project.cuh"
 #include "k_resident.cuh"
+#include "k_resident_deep.cuh"
 #include "ntcfd_common.cuh"
 
 using namespace ntcfd;
@@ -381,6 +382,42 @@ ResidentFn<Tc> resident_kernel(const Brick& b) {
     return resident_kernel_m<Tc, kResWide>(b);
 }
 
+// The resident kernel of a plan.
+template <class Tc>
+const void* resident_handle(const Brick& b) {
+    return b.deep ? (const void*)k_sor_deep<Tc, kResNT> : (const void*)resident_kernel<Tc>(b);
+}
+
+// The resident kernel's arguments for a solve, in the order of the plan's kernel.
+template <class Tc>
+struct ResidentArgs {
+    Geom g;
+    SorCoef<Tc> sc;
+    Brick br;
+    double* p;
+    const double* b;
+    Tc *dR, *dB;
+    const Tc *rdR, *rdB;
+    Ctl* ctl;
+    ResSync* sync;
+    unsigned long long* boxes;
+    double omega, zeta;
+    int itmax, cycle_len, check_every;
+    void* arg[17];
+    ResidentArgs(ntcfd_ctx* ctx, double* p_, const double* b_, double omega_, double zeta_, int itmax_, int cycle_,
+                 int check_)
+        : g(ctx->g), sc(sor_coef<Tc>(ctx)), br(ctx->brick), p(p_), b(b_), dR((Tc*)ctx->dR), dB((Tc*)ctx->dB),
+          rdR((const Tc*)ctx->rdR), rdB((const Tc*)ctx->rdB), ctl(ctx->ctl), sync(ctx->rsync), boxes(ctx->boxes),
+          omega(omega_), zeta(zeta_), itmax(itmax_), cycle_len(cycle_), check_every(check_) {
+        void* all[] = {&g, &sc, &br, &p, &b, &dR, &dB, &rdR, &rdB, &ctl, &sync, &boxes, &omega, &zeta, &itmax, &cycle_len,
+                       &check_every};
+        int k = 0;
+        for (int q = 0; q < 17; ++q)
+            if (!br.deep || (q != 4 && q != 7 && q != 8)) arg[k++] = all[q];   // no b, no rd
+    }
+    ResidentArgs(const ResidentArgs&) = delete;
+};
+
 // Brick plan of the resident SOR kernel: the split of the (j,k) rows into at
 // most (SM count) bricks of least estimated time per half-sweep, under the shared
 // memory limit (e of both colours for the brick and a one-row halo, plus d
@@ -391,7 +428,17 @@ ResidentFn<Tc> resident_kernel(const Brick& b) {
 // shared-memory words); rows without cached d and rd half as much again; the
 // hand-over between CTAs 1500.  So a grid of few rows runs in one CTA without any
 // hand-over: 12x10x8 takes 2.0 us a sweep (FP32) and 2.3 us (FP64) there against
-// 3.2 and 3.0 on 4 CTAs.  *us receives the time of a sweep by that estimate at 680
+// 3.2 and 3.0 on 4 CTAs.
+//
+// k_sor_deep, with one hand-over a sweep, has a cost of its own: 880 (FP64 950) for the
+// hand-over and the barriers, 187 (235) per turn of the warps over the rows of a colour,
+// fitted to sweeps of 1.6 to 7.6 us on 18 grids.  The other estimate reads 1 / 0.85 (FP32),
+// 1 / 0.76 (FP64) of the measured times of such rows, hence the factors.  So it takes the grids of
+// small bricks (12x10x8 FP64 1.6 us a sweep against 2.3, 40^3 2.6 against 3.3, 32x96x96 FP32 2.7
+// against 3.8, 64x96x96 3.75 against 4.9) and leaves larger FP64 bricks (40x100x100: 6.3 against
+// 6.0) and those whose extra arrays do not fit.
+//
+// *us receives the time of a sweep by that estimate at 680
 // clocks a microsecond (the measured times of 17 FP32 grids of 0.3 to 3.1 M cells lie
 // within 10% of it where d is cached; rows of less than 32 pairs take up to 1.6
 // times the estimate, wide ones 1.1).  Returns false when no plan fits one CTA per SM.
@@ -404,13 +451,14 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
     const long long per = kResNT / 32 * (mode == kResNarrow ? 2 * (32 / half) : 1);   // rows of a pass
     const double pass = (mode == kResNarrow ? 640.0 : 360.0 * ((half + 63) / 64)) * (sizeof(Tc) == 8 ? 1.7 : 1.0);
     double best = -1.0;
-    Brick bb{};
+    Brick bb{}, db{};
     size_t bsm = 0;
+    double deep = -1.0;
     for (int nbk = 1; nbk <= std::max(1, g.nz / 2) && nbk <= ctx->sm_count; ++nbk) {
         const int KB = (g.nz + nbk - 1) / nbk;
         for (int nbj = 1; nbj <= std::max(1, g.ny / 2) && nbj * nbk <= ctx->sm_count; ++nbj) {
             const int JB = (g.ny + nbj - 1) / nbj;
-            Brick b{nbj, nbk, JB, KB, mx, 0, 0, mode, 2 * (JB + KB) * half};
+            Brick b{nbj, nbk, JB, KB, mx, 0, 0, mode, 2 * (JB + KB) * half, 0};
             if (resident_smem<Tc>(b, g.nx) > limit) continue;
             // cache d, then rd, when they fit as well
             b.cache_d = 1;
@@ -426,10 +474,26 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
                 bb = b;
                 bsm = resident_smem<Tc>(b, g.nx);
             }
+            Brick d = b;
+            d.deep = 1;
+            d.inbox = deep_inbox_rows(d) * half;
+            if (mode != kResNarrow || nbj * nbk < 2 || deep_smem<Tc>(d) > limit) continue;
+            const long long turn = per / 2, red = rows + 2 * ((nbj > 1 ? KB : 0) + (nbk > 1 ? JB : 0));
+            const double turns = (double)((red + turn - 1) / turn + (rows + turn - 1) / turn);
+            const double dcost = sizeof(Tc) == 8 ? 950.0 + 235.0 * turns : 880.0 + 187.0 * turns;
+            if (deep < 0 || dcost < deep) {
+                deep = dcost;
+                db = d;
+            }
         }
     }
+    if (deep >= 0 && deep < (sizeof(Tc) == 8 ? 0.76 : 0.85) * best) {
+        best = deep;
+        bb = db;
+        bsm = deep_smem<Tc>(db);
+    }
     if (best < 0) return false;
-    auto kern = resident_kernel<Tc>(bb);
+    const void* kern = resident_handle<Tc>(bb);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -449,7 +513,7 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
     ctx->res_smem = bsm;
     ctx->res_grid = bb.nbj * bb.nbk;
     const double idle = half < 32 ? (32 - half) / 32.0 : 0.0;
-    *us = best / 680.0 * (mode == kResNarrow ? 1.0 + 0.8 * idle * idle : mode == kResWide ? 1.1 : 1.0);
+    *us = best / 680.0 * (bb.deep ? 1.0 : mode == kResNarrow ? 1.0 + 0.8 * idle * idle : mode == kResWide ? 1.1 : 1.0);
     return true;
 }
 
@@ -638,10 +702,9 @@ int add_step_nodes(ntcfd_ctx* ctx, cudaGraph_t G, int extra) {
                       (const double*)ctx->b, dR, dB, eR, eB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl,
                       (cudaGraphConditionalHandle)0, 0, ctx->rsync, 1, 0));
         dep = {n};
-        GK(add_kernel_ex(&n, G, dep, resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT),
-                         ctx->res_smem, true, g, sor_coef<Tc>(ctx), ctx->brick, ctx->p, (const double*)ctx->b,
-                         dR, dB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, ctx->rsync, ctx->boxes, P.omega,
-                         P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps));
+        ResidentArgs<Tc> ra(ctx, ctx->p, ctx->b, P.omega, P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps);
+        GK(add_cooperative(&n, G, dep, resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ctx->res_smem,
+                           ra.arg));
         dep = {n};
     } else if (ctx->march) {
         // the marching kernel runs the whole solve, after its barrier is cleared
@@ -832,11 +895,9 @@ int sor_solve_eager(ntcfd_ctx* ctx, double* p, const double* b, double zeta, int
         // one defect (starting the solve) and one launch that runs every cycle
         k_defect<Tc><<<g3, b3, 0, st>>>(g, ctx->scd, p, b, dR, dB, eR, eB, (const Tc*)ctx->rdR,
                                         (const Tc*)ctx->rdB, ctx->ctl, 0, 0, ctx->rsync, 1, 0);
-        void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&p, (void*)&b, (void*)&dR, (void*)&dB,
-                        (void*)&ctx->rdR, (void*)&ctx->rdB, (void*)&ctx->ctl, (void*)&ctx->rsync, (void*)&ctx->boxes,
-                        (void*)&omega, (void*)&zeta, (void*)&itmax, (void*)&ctx->cycle_len, (void*)&ctx->csweeps};
-        CK(cudaLaunchCooperativeKernel((const void*)resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid),
-                                       dim3(kResNT), args, ctx->res_smem, st));
+        ResidentArgs<Tc> ra(ctx, p, b, omega, zeta, itmax, ctx->cycle_len, ctx->csweeps);
+        CK(cudaLaunchCooperativeKernel(resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ra.arg,
+                                       ctx->res_smem, st));
         if (int rc = read_ctl()) return rc;
         CK(cudaGetLastError());
         return 0;
@@ -1085,12 +1146,9 @@ int time_kernels_t(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
             k_defect<Tc><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, pscratch, ctx->b, dR, dB, eR, eB,
                                                      (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, 0, 0,
                                                      ctx->rsync, 1, 0);
-            void* args[] = {(void*)&g, (void*)&sc, (void*)&ctx->brick, (void*)&pscratch, (void*)&ctx->b, (void*)&dR,
-                            (void*)&dB, (void*)&ctx->rdR, (void*)&ctx->rdB, (void*)&ctx->ctl, (void*)&ctx->rsync,
-                            (void*)&ctx->boxes, (void*)&P.omega, (void*)&kZeroZeta, (void*)sweeps, (void*)sweeps,
-                            (void*)&kOne};
-            cudaLaunchCooperativeKernel((const void*)resident_kernel<Tc>(ctx->brick), dim3(ctx->res_grid),
-                                        dim3(kResNT), args, ctx->res_smem, ctx->stream);
+            ResidentArgs<Tc> ra(ctx, pscratch, ctx->b, P.omega, 0.0, *sweeps, *sweeps, 1);
+            cudaLaunchCooperativeKernel(resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ra.arg,
+                                        ctx->res_smem, ctx->stream);
         };
         const int none = 0;
         float t0 = 0.0f;
