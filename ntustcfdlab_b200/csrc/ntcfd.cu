@@ -2347,9 +2347,9 @@ int adjoint_step(ntcfd_ctx* ctx, AdjBufs& A, const double* su, const double* sv,
     ab.lu = A.lu; ab.lv = A.lv; ab.lw = A.lw; ab.lp = A.lp;
     std::memcpy(ab.bc, P.bc, sizeof ab.bc);
     ab.gval = A.gval;
-    k_adj_bc_z<<<dim3((g.nx + 4 + 31) / 32, (g.ny + 4 + 7) / 8), dim3(32, 8), 0, st>>>(g, ab);
-    k_adj_bc_y<<<dim3((g.nx + 4 + 31) / 32, (g.nz + 4 + 7) / 8), dim3(32, 8), 0, st>>>(g, ab);
-    k_adj_bc_x<<<dim3((g.ny + 4 + 31) / 32, (g.nz + 4 + 7) / 8), dim3(32, 8), 0, st>>>(g, ab);
+    k_adj_bc<2><<<dim3((g.nx + 4 + 31) / 32, (g.ny + 4 + 1) / 2), dim3(32, 2), 0, st>>>(g, ab);
+    k_adj_bc<1><<<dim3((g.nx + 4 + 31) / 32, (g.nz + 4 + 1) / 2), dim3(32, 2), 0, st>>>(g, ab);
+    k_adj_bc<0><<<dim3((g.ny + 4 + 31) / 32, (g.nz + 4 + 1) / 2), dim3(32, 2), 0, st>>>(g, ab);
     k_adj_weights<<<g3, b3, 0, st>>>(g, guards, scaleD, scaleL, A.wD, A.wL);
     if (A.geta) {
         // u* of the step again (the forward predictor on the state before it), for u1
@@ -2597,9 +2597,9 @@ int adjoint_t(ntcfd_ctx* ctx, const ntcfd_adj_spec* sp, ntcfd_adj_result* res, d
         ab.lu = A.lu; ab.lv = A.lv; ab.lw = A.lw; ab.lp = A.lp;
         std::memcpy(ab.bc, P.bc, sizeof ab.bc);
         ab.gval = A.gval;
-        k_adj_bc_z<<<gbz, bbc, 0, st>>>(g, ab);
-        k_adj_bc_y<<<gby, bbc, 0, st>>>(g, ab);
-        k_adj_bc_x<<<gbx, bbc, 0, st>>>(g, ab);
+        k_adj_bc<2><<<gbz, bbc, 0, st>>>(g, ab);
+        k_adj_bc<1><<<gby, bbc, 0, st>>>(g, ab);
+        k_adj_bc<0><<<gbx, bbc, 0, st>>>(g, ab);
         CK(cudaGetLastError());
     }
     // ---- results
