@@ -45,8 +45,6 @@ constexpr int kSweepKpt = 4;
 constexpr int kResNT = 512;      // threads per CTA of the resident SOR kernel
 constexpr int kMixedCycle = 8;   // default FP32 sweeps per defect-correction cycle (mixed_cycle = 0)
 constexpr int kAdjQueued = 16;   // loop bodies an adjoint solve queues per host round trip (streaming)
-const double kZeroZeta = 0.0;
-const int kOne = 1;
 
 // The streaming half-sweep of a precision.  FP64 moves 40 B per cell and runs
 // closest to the HBM bandwidth in the column form (four planes per thread,
@@ -493,27 +491,31 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
         bsm = deep_smem<Tc>(db);
     }
     if (best < 0) return false;
-    const void* kern = resident_handle<Tc>(bb);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResNT, bsm) != cudaSuccess ||
-        per_sm < 1 || (long long)bb.nbj * bb.nbk > (long long)per_sm * ctx->sm_count) {
-        cudaGetLastError();
-        return false;
-    }
-    const size_t words = (size_t)bb.nbj * bb.nbk * 2 * bb.inbox * RingWord<Tc>::n;
-    if (words > ctx->box_words) {
-        if (dalloc(ctx, &ctx->boxes, words)) return false;
-        ctx->box_words = words;
-    }
     ctx->brick = bb;
     ctx->res_smem = bsm;
     ctx->res_grid = bb.nbj * bb.nbk;
     const double idle = half < 32 ? (32 - half) / 32.0 : 0.0;
     *us = best / 680.0 * (bb.deep ? 1.0 : mode == kResNarrow ? 1.0 + 0.8 * idle * idle : mode == kResWide ? 1.1 : 1.0);
+    return true;
+}
+
+// Takes the brick plan into use: the kernel's attributes and its inboxes.
+template <class Tc>
+bool use_resident(ntcfd_ctx* ctx) {
+    const Brick& b = ctx->brick;
+    const void* kern = resident_handle<Tc>(b);
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->res_smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResNT, ctx->res_smem) != cudaSuccess ||
+        per_sm < 1 || (long long)ctx->res_grid > (long long)per_sm * ctx->sm_count) {
+        cudaGetLastError();
+        return false;
+    }
+    const size_t words = (size_t)ctx->res_grid * 2 * b.inbox * RingWord<Tc>::n;
+    if (words > ctx->box_words) {
+        if (dalloc(ctx, &ctx->boxes, words)) return false;
+        ctx->box_words = words;
+    }
     return true;
 }
 
@@ -611,16 +613,17 @@ int choose_solve(ntcfd_ctx* ctx) {
     const int path = ctx->prm.sor_path;
     double tr = 0.0, tm = 0.0;
     MarchPlan mp;
-    ctx->march = false;
-    ctx->resident = path != NTCFD_SOR_STREAMING && plan_resident<Tc>(ctx, &tr);
+    ctx->march = ctx->resident = false;
+    const bool fits = path != NTCFD_SOR_STREAMING && plan_resident<Tc>(ctx, &tr);
     if (path == NTCFD_SOR_RESIDENT) {
+        ctx->resident = fits && use_resident<Tc>(ctx);
         if (!ctx->resident) return fail(ctx, NTCFD_EINVAL, "the resident SOR kernel does not fit this grid on this device");
         return 0;
     }
-    if (ctx->resident && sizeof(Tc) == 8) return 0;
-    if (!plan_march<Tc>(ctx, &mp, &tm) || (ctx->resident && tm > 0.95 * tr)) return 0;
-    ctx->march = use_march<Tc>(ctx, mp);
-    ctx->resident = ctx->resident && !ctx->march;
+    const bool marches = plan_march<Tc>(ctx, &mp, &tm);
+    if (fits && !(marches && sizeof(Tc) == 4 && tm <= 0.95 * tr)) ctx->resident = use_resident<Tc>(ctx);
+    if (!ctx->resident && marches) ctx->march = use_march<Tc>(ctx, mp);
+    if (!ctx->resident && !ctx->march && fits) ctx->resident = use_resident<Tc>(ctx);
     return 0;
 }
 
