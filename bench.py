@@ -282,7 +282,7 @@ def roofline(s, case, path, reps=20):
     grid from an ncu capture (profiles/sor_traffic.json).  `bound` follows
     from it: a kernel whose DRAM traffic is well below its algorithmic bytes
     works out of shared memory and L2, so the HBM roofline does not bind it
-    ("on-chip"; the resident kernel is then bound by its grid barriers and
+    ("on-chip"; the resident kernel is then bound by its hand-overs between CTAs and
     instruction issue); otherwise "hbm".  Both fractions are reported: the
     algorithmic one (`frac`) and the DRAM one (`dram_frac`).
 
