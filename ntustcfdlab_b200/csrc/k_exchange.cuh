@@ -16,7 +16,7 @@ constexpr unsigned int kRingPolls = 4000000u;    // polls of one word before giv
 
 // Device memory of the exchange (one per context).  k_defect zeroes all but seq.
 struct ResSync {
-    GridBar bar;                     // the closing barrier's word, the error flag
+    GridBar bar;                     // the grid barrier's words, the error flag
     unsigned long long cnt[2][4];    // [colour][sweep & 3]: arrivals, and verdicts in the high half
     unsigned long long last;         // max |change| of the last sweep
     unsigned int seq;                // sequence number of the last half-sweep of earlier launches
@@ -63,15 +63,6 @@ struct RingWord<double> {
         asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
     }
 };
-
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_add_relaxed(unsigned long long* p, unsigned long long v) {
-    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 
 // Waits until the counter's low half reaches target; false when it gives up.
 __device__ __forceinline__ bool count_wait(const unsigned long long* c, unsigned int target, int* err,

@@ -659,7 +659,7 @@ template <class Tc, int HP>
 __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_constant__ MarchArgs<Tc> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_flag, s_nan[2];
-    __shared__ unsigned int s_hi;
+    __shared__ unsigned int s_over;               // CTAs above zeta, 2^20 per one that met a NaN, of a sweep
     __shared__ unsigned long long s_max[kMarchNT / 32 + 1];
     __shared__ MarchBars s_bars;
     __shared__ bool s_lost;
@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
         const int bk = blockIdx.x / a.nbj;
         steps = brick_start(bk + 1, a.g.nz, a.nbk) - brick_start(bk, a.g.nz, a.nbk) + 2;
     }
-    unsigned int nbar = 0, hi_prev = 0u;
+    GridPlace at;
     const unsigned int nblocks = gridDim.x;
-    bool failed = !grid_sync(&a.sync->bar, nbar, nblocks, &s_flag);
+    bool failed = !grid_sync(&a.sync->bar, at, nblocks, &s_flag);
 
     int done = 0, done_c = 0, cycles = 0, cur = 0;    // cur: the buffer that holds e
     bool conv = false, nonfinite = false, tested = false;
@@ -717,13 +717,12 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
                 failed = true;
                 break;
             }
-            if (!grid_sync(&a.sync->bar, nbar, nblocks, &s_flag,
-                           (any ? 1u : 0u) + (tid == 0 && s_nan[par] ? 1u << 20 : 0u), &s_hi)) {
+            if (!grid_sync(&a.sync->bar, at, nblocks, &s_flag,
+                           (any ? 1u : 0u) + (tid == 0 && s_nan[par] ? 1u << 20 : 0u), &s_over)) {
                 failed = true;
                 break;
             }
-            const unsigned int over = s_hi - hi_prev;   // CTAs above zeta, 2^20 per one that met a NaN
-            hi_prev = s_hi;
+            const unsigned int over = s_over;
             chs = cb;
             done_c = s + 1;
             if (a.check_every == 1 || ik >= a.itmax || ik % a.check_every == 0) {
@@ -739,7 +738,7 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
         if (failed || conv || nonfinite || done_c < a.cycle_len || done >= a.itmax) break;
         march_restart<Tc, HP>(a, &s_bars, cur, n, &s_lost);
         n += steps - 2;
-        if (!grid_sync(&a.sync->bar, nbar, nblocks, &s_flag) || s_lost) failed = true;
+        if (!grid_sync(&a.sync->bar, at, nblocks, &s_flag) || s_lost) failed = true;
     }
     if (!failed && done > 0) march_correct<Tc>(a, cur);
     double last = 0.0;
@@ -756,7 +755,7 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
             for (int w = 0; w < (int)blockDim.x / 32; ++w) m = s_max[w] > m ? s_max[w] : m;
             atomicMax(&a.sync->last, m);
         }
-        if (!grid_sync(&a.sync->bar, nbar, nblocks, &s_flag)) failed = true;
+        if (!grid_sync(&a.sync->bar, at, nblocks, &s_flag)) failed = true;
         else if (tid == 0) last = __longlong_as_double((long long)ld_relaxed(&a.sync->last));
     }
     if (blockIdx.x == 0 && tid == 0) {
@@ -775,7 +774,7 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
 
 // Start of a solve of the marching kernel: its barrier and slot cleared.
 __global__ void k_march_begin(ResSync* rs) {
-    rs->bar.word = 0ULL;
+    rs->bar.word[0] = rs->bar.word[1] = 0ULL;
     rs->bar.err = 0;
     rs->last = 0ULL;
 }

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) k_defect(Geom g, SorCoef<double> sc, cons
         ctl->inner = 0;
         if (in_graph) cudaGraphSetConditional(inner, 1u);
         if (rs) {                       // the resident kernel's counters (not its sequence number)
-            rs->bar.word = 0ULL;
+            rs->bar.word[0] = rs->bar.word[1] = 0ULL;
             rs->bar.err = 0;
             for (int q = 0; q < 4; ++q) rs->cnt[0][q] = rs->cnt[1][q] = 0ULL;
             rs->last = 0ULL;

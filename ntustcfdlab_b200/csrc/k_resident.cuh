@@ -740,8 +740,8 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
             else last = __longlong_as_double((long long)widen_bits(b2));
         }
         if (multi) {
-            unsigned int nbar = 0;
-            if (!grid_sync(&sync->bar, nbar, nblocks, &s_flag)) failed = true;
+            GridPlace at;
+            if (!grid_sync(&sync->bar, at, nblocks, &s_flag)) failed = true;
             else if (tid == 0) last = __longlong_as_double((long long)ld_relaxed(&sync->last));
         }
     }

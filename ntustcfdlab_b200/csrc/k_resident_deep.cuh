@@ -404,8 +404,8 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
             for (int q = 0; q < NWARP; ++q) b2 = s_red_max[q] > b2 ? s_red_max[q] : b2;
             atomicMax(&sync->last, widen_bits(b2));
         }
-        unsigned int nbar = 0;
-        if (!grid_sync(&sync->bar, nbar, nblocks, &s_flag)) failed = true;
+        GridPlace at;
+        if (!grid_sync(&sync->bar, at, nblocks, &s_flag)) failed = true;
         else if (tid == 0) last = __longlong_as_double((long long)ld_relaxed(&sync->last));
     }
     if (blockIdx.x == 0 && tid == 0) {
