@@ -701,6 +701,12 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
     unsigned long long chs = 0ull;                    // this thread's max |change| of the last sweep
 
     auto above = [&](unsigned long long b) { return !(__longlong_as_double((long long)b) <= a.zeta); };
+    // Whether a wait of this CTA gave up, after a CTA barrier: it then leaves without
+    // arriving at the grid barrier, and the error flag takes the others out of it.
+    auto lost = [&]() {
+        if (s_lost && tid == 0) atomicExch(&a.sync->bar.err, 1);
+        return s_lost;
+    };
 
     while (!failed) {
         done_c = 0;
@@ -712,13 +718,8 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
             cur ^= 1;
             if (cb >= kInfBits) s_nan[par] = 1;
             const int any = __syncthreads_or(above(cb));
-            if (s_lost) {
-                if (tid == 0) atomicExch(&a.sync->bar.err, 1);
-                failed = true;
-                break;
-            }
-            if (!grid_sync(&a.sync->bar, at, nblocks, &s_flag,
-                           (any ? 1u : 0u) + (tid == 0 && s_nan[par] ? 1u << 20 : 0u), &s_over)) {
+            if (lost() || !grid_sync(&a.sync->bar, at, nblocks, &s_flag,
+                                     (any ? 1u : 0u) + (tid == 0 && s_nan[par] ? 1u << 20 : 0u), &s_over)) {
                 failed = true;
                 break;
             }
@@ -738,7 +739,8 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
         if (failed || conv || nonfinite || done_c < a.cycle_len || done >= a.itmax) break;
         march_restart<Tc, HP>(a, &s_bars, cur, n, &s_lost);
         n += steps - 2;
-        if (!grid_sync(&a.sync->bar, at, nblocks, &s_flag) || s_lost) failed = true;
+        __syncthreads();
+        if (lost() || !grid_sync(&a.sync->bar, at, nblocks, &s_flag)) failed = true;
     }
     if (!failed && done > 0) march_correct<Tc>(a, cur);
     double last = 0.0;

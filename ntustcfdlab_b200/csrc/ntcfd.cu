@@ -1635,7 +1635,7 @@ int records_to_info(ntcfd_ctx* ctx, const StepRec* rec, int nsteps, ntcfd_step_i
             I.aoa = aoa ? aoa[s] : 0.0;
         }
     }
-    if (status == NTCFD_ETIMEOUT) fail(ctx, status, "the resident SOR kernel's grid barrier gave up waiting");
+    if (status == NTCFD_ETIMEOUT) fail(ctx, status, "a wait of the SOR solve's kernel gave up");
     else if (status == NTCFD_ENONFINITE) fail(ctx, status, "non-finite value in the SOR solve");
     else if (status == NTCFD_NOT_CONVERGED) fail(ctx, status, "SOR stopped at itmax in at least one step");
     return status;
@@ -2388,7 +2388,7 @@ int adjoint_step(ntcfd_ctx* ctx, AdjBufs& A, const double* su, const double* sv,
         CK(cudaEventElapsedTime(&sms, A.e0, A.e1));
         A.solve_ms += sms;
         A.solves += 1;
-        if (h.timeout) return fail(ctx, NTCFD_ETIMEOUT, "the resident SOR kernel's grid barrier gave up waiting");
+        if (h.timeout) return fail(ctx, NTCFD_ETIMEOUT, "a wait of the SOR solve's kernel gave up");
         if (h.nonfinite) return fail(ctx, NTCFD_ENONFINITE, "non-finite value in an adjoint SOR solve");
         *sweeps += h.ik;
         if (!h.converged) *unconverged += 1;
