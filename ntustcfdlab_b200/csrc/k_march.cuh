@@ -323,6 +323,19 @@ struct MarchPos {
     }
 };
 
+// The copying thread's end of a march of `issued` steps, the last of them before pos: it waits
+// (with the limit of every wait) until its last copies have landed, also where the march was
+// given up, so that no copy is in flight when the CTA leaves.  In a march that ran through, the
+// updating warps have waited for the same copies.
+__device__ __forceinline__ bool march_drain(MarchBars* bars, MarchPos pos, int issued) {
+    bool ok = true;
+    for (int q = min(issued, kMarchAhead + 1); q > 0; --q) {
+        pos = pos.prev();
+        ok = mbar_wait(bars->full + pos.slot, pos.lap) && ok;
+    }
+    return ok;
+}
+
 // The restart of a correction cycle: p += e (buffer cur) and d = the FP64 defect of
 // p + e (defect_update), in a march with the sweep's copies: e of plane k+1 and d
 // of plane k.
@@ -353,9 +366,9 @@ __device__ __noinline__ void march_restart(const MarchArgs<Tc>& a, MarchBars* ba
         bool ok = true;
         if (tid == nt) {
             constexpr unsigned int w = sizeof(Tc);
-            int ef = 1;
+            int ef = 1, issued = 0;
             fence_bulk();
-            for (int k = ka; k <= kb && ok; ++k) {
+            for (int k = ka; k <= kb; ++k, ++issued) {
                 if (k > ka + D) ok = mbar_wait(bars->done + pos.slot, pos.lap ^ 1u);
                 if (!ok) break;
                 const int sR = Ri + tile0 + k * ps, sB = sR + a.elems, sd = Di + tile0 + k * ps;
@@ -373,7 +386,7 @@ __device__ __noinline__ void march_restart(const MarchArgs<Tc>& a, MarchBars* ba
                 ef = wrap(ef, D + 2);
                 pos.next();
             }
-            if (!ok) *lost = true;
+            if (!march_drain(bars, pos, issued) || !ok) *lost = true;
         }
         return;
     }
@@ -518,9 +531,9 @@ __device__ __noinline__ unsigned long long march_sweep(const MarchArgs<Tc>& a, M
         if (tid == nt) {
             // step k's copies; a cycle's first sweep copies a plane of zeros (k = -1) for e
             constexpr unsigned int w = sizeof(Tc);
-            int bf = 1;
+            int bf = 1, issued = 0;
             fence_bulk();
-            for (int k = ka - 1; k <= kb + 1 && ok; ++k) {
+            for (int k = ka - 1; k <= kb + 1; ++k, ++issued) {
                 if (k > ka - 1 + D) ok = mbar_wait(bars->done + pos.slot, pos.lap ^ 1u);
                 if (!ok) break;
                 const int sB = Bi + tile0 + (first ? -1 : k + 1) * ps, sR = Ri + tile0 + (first ? -1 : k) * ps;
@@ -536,7 +549,7 @@ __device__ __noinline__ unsigned long long march_sweep(const MarchArgs<Tc>& a, M
                 bf = wrap(bf, D + 2);
                 pos.next();
             }
-            if (!ok) *lost = true;
+            if (!march_drain(bars, pos, issued) || !ok) *lost = true;
         }
         return 0ull;
     }
