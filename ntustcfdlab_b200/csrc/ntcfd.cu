@@ -499,13 +499,23 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
     return true;
 }
 
+// Lets a kernel take `smem` bytes of dynamic shared memory.  The attribute belongs to the
+// kernel, not to a context: every context sets it to the device's limit, so that none lowers it
+// below another's plan.
+bool allow_smem(const ntcfd_ctx* ctx, const void* kern, size_t smem) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || smem + fa.sharedSizeBytes > ctx->smem_optin) return false;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(ctx->smem_optin - fa.sharedSizeBytes)) == cudaSuccess;
+}
+
 // Takes the brick plan into use: the kernel's attributes and its inboxes.
 template <class Tc>
 bool use_resident(ntcfd_ctx* ctx) {
     const Brick& b = ctx->brick;
     const void* kern = resident_handle<Tc>(b);
     int per_sm = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->res_smem) != cudaSuccess ||
+    if (!allow_smem(ctx, kern, ctx->res_smem) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResNT, ctx->res_smem) != cudaSuccess ||
         per_sm < 1 || (long long)ctx->res_grid > (long long)per_sm * ctx->sm_count) {
         cudaGetLastError();
@@ -582,7 +592,7 @@ bool use_march(ntcfd_ctx* ctx, const MarchPlan& m) {
     int per_sm = 0;
     size_t free_b = 0, total = 0;
     const void* kern = march_kernel<Tc>(m.HP);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.smem) != cudaSuccess ||
+    if (!allow_smem(ctx, kern, m.smem) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, m.nt, m.smem) != cudaSuccess ||
         (long long)m.nbj * m.nbk > (long long)per_sm * ctx->sm_count ||
         (!ctx->mf && cudaMemGetInfo(&free_b, &total) != cudaSuccess)) {
