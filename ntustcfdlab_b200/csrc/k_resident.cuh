@@ -38,7 +38,8 @@
 //
 // A lane updates two cells at a time with every load issued before any
 // store: cells t and t + 32 of one row (rows of at most 64 cells per colour,
-// or in 64-cell chunks for wider rows), or, in the NARROW instance (rows of
+// or in 64-cell chunks for wider rows; one cell where a last chunk has 32 or fewer: 160x120x120
+// FP64 17.5 us a sweep against 19.9 with two throughout), or, in the NARROW instance (rows of
 // at most 32 cells per colour), t of two rows.  The row's parity r is a
 // template argument of the update, so the east/west neighbours and the second
 // cell are immediate offsets of one address.  Loads always read inside the
@@ -57,8 +58,11 @@
 
 namespace ntcfd {
 
-// Row shapes of k_sor_resident (Brick::mode).
-enum { kResNarrow = 0, kResWide1 = 1, kResWide = 2 };
+// Row shapes of k_sor_resident (Brick::mode): several rows side by side on a warp's lanes; rows of 33
+// to 64 cells per colour; a warp per longer row; a warp per 64-cell chunk of a longer row, for bricks of
+// few rows (1000x20x16, three or four rows of eight chunks a CTA: FP32 6.7 us a sweep against 7.6 by
+// rows), which may be one row thick.
+enum { kResNarrow = 0, kResWide1 = 1, kResWide = 2, kResLong = 3 };
 
 struct Brick {
     int nbj, nbk;    // bricks along j and k
@@ -66,7 +70,7 @@ struct Brick {
     int mx;          // colour-split row length (compact index m = 0..mx-1)
     int cache_d;     // 1: d of the brick lives in shared memory too
     int cache_rd;    // 1: rd of the brick lives in shared memory too
-    int mode;        // kResNarrow, kResWide1 or kResWide (res_mode(nx))
+    int mode;        // kResNarrow, kResWide1 or kResWide (res_mode(nx)); kResLong: wide rows by chunks
     int inbox;       // ring words per CTA and colour
     int deep;        // 1: k_sor_deep (k_resident_deep.cuh)
 };
@@ -77,6 +81,15 @@ __host__ __device__ inline int res_mode(int nx) {
     return most <= 32 ? kResNarrow : most <= 64 ? kResWide1 : kResWide;
 }
 
+// Rows of a brick with a neighbour, at most.
+__host__ __device__ inline int res_edge_rows(int JB, int KB) {
+    return JB > 2 && KB > 2 ? 2 * (JB + KB) - 4 : JB * KB;
+}
+// Bytes of the edge rows' places in the neighbours' inboxes.
+inline size_t resident_places(const Brick& b) {
+    return (size_t)res_edge_rows(b.JB, b.KB) * (b.mode == kResLong ? 16 : 8);
+}
+
 // Dynamic shared memory of k_sor_resident for a brick plan.
 template <class Tc>
 inline size_t resident_smem(const Brick& b, int nx) {
@@ -84,12 +97,12 @@ inline size_t resident_smem(const Brick& b, int nx) {
     const size_t brick = (size_t)b.JB * b.KB * b.mx;
     const size_t arrays = sizeof(Tc) * (2 * tile + 2 * (size_t)(nx + 4) + 2 * (size_t)(b.JB + b.KB) +
                                         (b.cache_d ? 2 * brick : 0) + (b.cache_rd ? 2 * brick : 0));
-    // + row table (int4 offsets, four coefficients and two inbox places per row), + the
-    // ring list (int2 per ring row), + slack: the loads of a lane past a row's last cell may
+    // + row table (int4 offsets and four coefficients per row), + the ring list (int2 per
+    // ring row), + the edge rows' places, + slack: the loads of a lane past a row's last cell may
     // reach up to 64 elements beyond the tiles
     const size_t rows = (size_t)b.JB * b.KB;
-    return ((arrays + 15) & ~size_t(15)) + rows * (16 + 4 * sizeof(Tc) + 8) + 2 * (size_t)(b.JB + b.KB) * 8 +
-           64 * sizeof(Tc);
+    return ((arrays + 15) & ~size_t(15)) + rows * (16 + 4 * sizeof(Tc)) + 2 * (size_t)(b.JB + b.KB) * 8 +
+           resident_places(b) + 64 * sizeof(Tc);
 }
 
 // ring words a thread holds in flight
@@ -128,6 +141,7 @@ struct ResRow {
     Tc cN, cS, cF, cB;
     int par;          // (j + k) & 1 of the row
     unsigned long long *pubA, *pubB;   // an edge row's words in its neighbours' inboxes (t = 0; null: none)
+    unsigned long long *pubC, *pubD;   // (FOUR)
 };
 
 // The loaded operands of one cell.
@@ -166,7 +180,7 @@ __device__ __forceinline__ ResIn<Tc> res_load(const ResRow<Tc>& w, int t, int m,
 // sweep against 8.4 with rd from L2 on 100x150x150 FP32, 12.6 against 13.6 on 33x150x220
 // FP64.  Where d comes from L2 as well, rd does too (formed: 64x128x256 FP64 13.0 us
 // against 12.4).
-template <class Tc, bool EDGE, bool FORM, class B>
+template <class Tc, bool EDGE, bool FORM, bool FOUR, class B>
 __device__ __forceinline__ void res_finish(const ResIn<Tc>& x, const ResRow<Tc>& w, int t, int m, Tc cE, Tc cW, Tc om,
                                            bool ok, bool ring, unsigned int seq, B& ch) {
     Tc e1;
@@ -183,6 +197,8 @@ __device__ __forceinline__ void res_finish(const ResIn<Tc>& x, const ResRow<Tc>&
         const Tc v = ok ? e1 : Tc(0);
         if (ring && w.pubA) Word::store(w.pubA + t * Word::n, v, seq);
         if (ring && w.pubB) Word::store(w.pubB + t * Word::n, v, seq);
+        if (FOUR && ring && w.pubC) Word::store(w.pubC + t * Word::n, v, seq);
+        if (FOUR && ring && w.pubD) Word::store(w.pubD + t * Word::n, v, seq);
     }
 }
 
@@ -225,13 +241,14 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     Tc* const arrays_end = CR ? R1 + brick : (CD ? D1 + brick : D0);
     // row table: per row of the brick, in sweep order (edge rows first), the tile row
     // start, the brick row start of d/rd, the global colour-split row start and
-    // (j+k)&1; the row's cN, cS, cF, cB; its places in the neighbours' inboxes.  Then the
-    // ring: per row of a neighbour brick (inbox order) its tile row start and (j+k)&1.
+    // (j+k)&1; the row's cN, cS, cF, cB; of the edge rows their places in the neighbours'
+    // inboxes.  Then the ring: per row of a neighbour brick (inbox order) its tile row start and (j+k)&1.
     const size_t toff = ((size_t)((unsigned char*)arrays_end - smem_raw) + 15) & ~size_t(15);
     int4* const rowT = reinterpret_cast<int4*>(smem_raw + toff);
     Tc* const rowC = reinterpret_cast<Tc*>(rowT + JB * KB);
-    int2* const pubT = reinterpret_cast<int2*>(rowC + 4 * JB * KB);
-    int2* const ringT = pubT + JB * KB;
+    using Places = std::conditional_t<MODE == kResLong, int4, int2>;
+    Places* const pubT = reinterpret_cast<Places*>(rowC + 4 * JB * KB);
+    int2* const ringT = reinterpret_cast<int2*>(pubT + res_edge_rows(JB, KB));
     constexpr int NWARP = NT / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tid = threadIdx.x;
@@ -291,19 +308,19 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
         rowC[4 * er + 1] = sc.cS[j];
         rowC[4 * er + 2] = sc.cF[k];
         rowC[4 * er + 3] = sc.cB[k];
+        if (er >= ne) continue;
         // the row's ring row in a neighbour: at most one along j and one along k (a brick
         // that has neighbours on both sides of a direction is two rows thick or more)
-        int pj = -1, pk = -1;
-        if (jl == 1 && jlo)                    // the j-high face of brick bj - 1
-            pj = (int)(blockIdx.x - 1) * 2 * br.inbox + ((bj > 1 ? nk : 0) + kl - 1) * nown1;
-        else if (jl == nj && jhi)              // the j-low face of brick bj + 1
-            pj = (int)(blockIdx.x + 1) * 2 * br.inbox + (kl - 1) * nown1;
-        if (kl == 1 && klo)                    // the k-high face of brick bk - 1
-            pk = (int)(blockIdx.x - br.nbj) * 2 * br.inbox +
-                 ((jlo ? nkl : 0) + (jhi ? nkl : 0) + (bk > 1 ? nj : 0) + jl - 1) * nown1;
-        else if (kl == nk && khi)              // the k-low face of brick bk + 1
-            pk = (int)(blockIdx.x + br.nbj) * 2 * br.inbox + ((jlo ? nkh : 0) + (jhi ? nkh : 0) + jl - 1) * nown1;
-        pubT[er] = pj >= 0 ? make_int2(pj, pk) : make_int2(pk, -1);
+        auto place = [&](int cta, int ring_row) { return cta * 2 * br.inbox + ring_row * nown1; };
+        const int me = (int)blockIdx.x;
+        const bool toJl = jl == 1 && jlo, toJh = jl == nj && jhi, toKl = kl == 1 && klo, toKh = kl == nk && khi;
+        const int pJl = place(me - 1, (bj > 1 ? nk : 0) + kl - 1);       // the j-high face of brick bj - 1
+        const int pJh = place(me + 1, kl - 1);                           // the j-low face of brick bj + 1
+        const int pKl = place(me - br.nbj, (jlo ? nkl : 0) + (jhi ? nkl : 0) + (bk > 1 ? nj : 0) + jl - 1);
+        const int pKh = place(me + br.nbj, (jlo ? nkh : 0) + (jhi ? nkh : 0) + jl - 1);
+        const int pj = toJl ? pJl : toJh ? pJh : -1, pk = toKl ? pKl : toKh ? pKh : -1;
+        if constexpr (MODE == kResLong) pubT[er] = make_int4(toJl ? pJl : -1, toJh ? pJh : -1, toKl ? pKl : -1, toKh ? pKh : -1);
+        else pubT[er] = pj >= 0 ? make_int2(pj, pk) : make_int2(pk, -1);
     }
     if (tid == 0) {
         s_fail[0] = s_fail[1] = s_nan[0] = s_nan[1] = 0;
@@ -342,8 +359,8 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int i = 2 * (lt + 32 * h) + 2 - r;
-            cEr[r][h] = MODE == kResWide ? Tc(0) : cEs[min(i, g.nx + 2)];
-            cWr[r][h] = MODE == kResWide ? Tc(0) : cWs[min(i, g.nx + 2)];
+            cEr[r][h] = MODE >= kResWide ? Tc(0) : cEs[min(i, g.nx + 2)];
+            cWr[r][h] = MODE >= kResWide ? Tc(0) : cWs[min(i, g.nx + 2)];
         }
 
     const unsigned int nblocks = gridDim.x;
@@ -522,6 +539,8 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     };
 
     // ---- one half-sweep of colour c over rows [e0r, e1r) (edge rows: EDGE)
+    const int nch = (nown1 + 63) / 64;                            // chunks of a row (kResLong)
+    const int row0 = warp / nch, chunk0 = warp - row0 * nch, rowstep = NWARP / nch, chunkstep = NWARP - rowstep * nch;
     auto rows_pass = [&](auto edge_tag, int c, int e0r, int e1r, unsigned int seq, B& ch) {
         constexpr bool EDGE = decltype(edge_tag)::value;
         Tc* const W = c ? S1 : S0;
@@ -548,9 +567,13 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
             }
             w.par = rt.w;
             if (EDGE) {
-                const int2 pb = pubT[er];
+                const Places pb = pubT[er];
                 w.pubA = pb.x >= 0 ? Ec + (size_t)pb.x * Word::n : nullptr;
                 w.pubB = pb.y >= 0 ? Ec + (size_t)pb.y * Word::n : nullptr;
+                if constexpr (MODE == kResLong) {
+                    w.pubC = pb.z >= 0 ? Ec + (size_t)pb.z * Word::n : nullptr;
+                    w.pubD = pb.w >= 0 ? Ec + (size_t)pb.w * Word::n : nullptr;
+                }
             }
             return w;
         };
@@ -565,35 +588,57 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
                 const int mA = lt + 2 - rA, mB = lt + 2 - rB;
                 const ResIn<Tc> xA = res_load<Tc, CD, CR>(wA, lt, mA, mx, plane);
                 const ResIn<Tc> xB = res_load<Tc, CD, CR>(wB, lt, mB, mx, plane);
-                res_finish<Tc, EDGE, CD && !CR>(xA, wA, lt, mA, rA ? cEr[1][0] : cEr[0][0], rA ? cWr[1][0] : cWr[0][0], om,
+                res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xA, wA, lt, mA, rA ? cEr[1][0] : cEr[0][0], rA ? cWr[1][0] : cWr[0][0], om,
                                      inA && lt < (rA ? nown1 : nown0), inA, seq, ch);
-                res_finish<Tc, EDGE, CD && !CR>(xB, wB, lt, mB, rB ? cEr[1][0] : cEr[0][0], rB ? cWr[1][0] : cWr[0][0], om,
+                res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xB, wB, lt, mB, rB ? cEr[1][0] : cEr[0][0], rB ? cWr[1][0] : cWr[0][0], om,
                                      inB && lt < (rB ? nown1 : nown0), inB, seq, ch);
             }
-        } else {
+        } else if constexpr (MODE == kResWide1) {
             for (int er = e0r + warp; er < e1r; er += NWARP) {
                 const ResRow<Tc> w = row_of(er);
                 const int r = (w.par ^ c) & 1;
                 const int nown = r ? nown1 : nown0;
-                if constexpr (MODE == kResWide1) {
-                    // cells t = lane (always in the row: it holds more than 32) and lane + 32
-                    const int m = lane + 2 - r;
-                    const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, lane, m, mx, plane);
-                    const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, lane + 32, m + 32, mx, plane);
-                    res_finish<Tc, EDGE, CD && !CR>(xA, w, lane, m, r ? cEr[1][0] : cEr[0][0], r ? cWr[1][0] : cWr[0][0], om, true, true,
-                                         seq, ch);
-                    res_finish<Tc, EDGE, CD && !CR>(xB, w, lane + 32, m + 32, r ? cEr[1][1] : cEr[0][1], r ? cWr[1][1] : cWr[0][1], om,
-                                         lane + 32 < nown, lane + 32 < nown1, seq, ch);
-                } else {
-                    for (int t0 = 0; t0 < nown1; t0 += 64) {
-                        const int tA = t0 + lane, m = tA + 2 - r;
-                        const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, tA, m, mx, plane);
-                        const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, tA + 32, m + 32, mx, plane);
-                        const int iA = min(2 * tA + 2 - r, g.nx + 2), iB = min(iA + 64, g.nx + 2);
-                        const Tc eA = cEs[iA], wA = cWs[iA], eB = cEs[iB], wB = cWs[iB];
-                        res_finish<Tc, EDGE, CD && !CR>(xA, w, tA, m, eA, wA, om, tA < nown, tA < nown1, seq, ch);
-                        res_finish<Tc, EDGE, CD && !CR>(xB, w, tA + 32, m + 32, eB, wB, om, tA + 32 < nown, tA + 32 < nown1, seq, ch);
+                // cells t = lane (always in the row: it holds more than 32) and lane + 32
+                const int m = lane + 2 - r;
+                const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, lane, m, mx, plane);
+                const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, lane + 32, m + 32, mx, plane);
+                res_finish<Tc, EDGE, CD && !CR, false>(xA, w, lane, m, r ? cEr[1][0] : cEr[0][0], r ? cWr[1][0] : cWr[0][0], om, true, true,
+                                     seq, ch);
+                res_finish<Tc, EDGE, CD && !CR, false>(xB, w, lane + 32, m + 32, r ? cEr[1][1] : cEr[0][1], r ? cWr[1][1] : cWr[0][1], om,
+                                     lane + 32 < nown, lane + 32 < nown1, seq, ch);
+            }
+        } else {
+            // the cells t0 + lane, and with `two` t0 + 32 + lane, of a row
+            auto chunk = [&](auto two, const ResRow<Tc>& w, int t0) __attribute__((always_inline)) {
+                constexpr bool TWO = decltype(two)::value;
+                const int r = (w.par ^ c) & 1;
+                const int nown = r ? nown1 : nown0;
+                const int tA = t0 + lane, m = tA + 2 - r;
+                const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, tA, m, mx, plane);
+                ResIn<Tc> xB;
+                if (TWO) xB = res_load<Tc, CD, CR>(w, tA + 32, m + 32, mx, plane);
+                const int iA = min(2 * tA + 2 - r, g.nx + 2), iB = min(iA + 64, g.nx + 2);
+                const Tc eA = cEs[iA], wA = cWs[iA], eB = cEs[iB], wB = cWs[iB];
+                res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xA, w, tA, m, eA, wA, om, tA < nown, tA < nown1, seq, ch);
+                if (TWO) res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xB, w, tA + 32, m + 32, eB, wB, om, tA + 32 < nown, tA + 32 < nown1, seq, ch);
+            };
+            if constexpr (MODE == kResLong) {
+                // a warp per 64-cell chunk of a row
+                int q = chunk0;
+                for (int er = e0r + row0; er < e1r; er += rowstep) {
+                    chunk(std::true_type{}, row_of(er), 64 * q);
+                    if ((q += chunkstep) >= nch) {
+                        q -= nch;
+                        ++er;
                     }
+                }
+            } else {
+                // a warp per row; of a last chunk of 32 cells or fewer only the first half
+                for (int er = e0r + warp; er < e1r; er += NWARP) {
+                    const ResRow<Tc> w = row_of(er);
+                    int t0 = 0;
+                    for (; t0 + 32 < nown1; t0 += 64) chunk(std::true_type{}, w, t0);
+                    if (t0 < nown1) chunk(std::false_type{}, w, t0);
                 }
             }
         }

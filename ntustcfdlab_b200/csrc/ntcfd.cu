@@ -377,6 +377,7 @@ template <class Tc>
 ResidentFn<Tc> resident_kernel(const Brick& b) {
     if (b.mode == kResNarrow) return resident_kernel_m<Tc, kResNarrow>(b);
     if (b.mode == kResWide1) return resident_kernel_m<Tc, kResWide1>(b);
+    if (b.mode == kResLong) return resident_kernel_m<Tc, kResLong>(b);
     return resident_kernel_m<Tc, kResWide>(b);
 }
 
@@ -417,16 +418,27 @@ struct ResidentArgs {
 };
 
 // Brick plan of the resident SOR kernel: the split of the (j,k) rows into at
-// most (SM count) bricks of least estimated time per half-sweep, under the shared
+// most (SM count) bricks of least estimated time per sweep, under the shared
 // memory limit (e of both colours for the brick and a one-row halo, plus d
-// when it also fits).  Bricks with a neighbour are two rows thick or more.
-// The estimate, in clocks: a pass of the warps over the interior rows takes about
-// 360 (one row a warp; 640 for the narrow form's two slots, each of several rows),
+// when it also fits).  Bricks with a neighbour are two rows thick or more, since a row then goes to
+// two neighbours at most, except those of kResLong.
+//
+// The estimate, in units of 1/680 us of a sweep: a turn of the warps over the interior rows takes
+// 360 (one row or 64-cell chunk a warp; 640 for the narrow form's two slots, each of several rows),
 // over the edge rows, which publish, 1.6 times that, FP64 1.7 times more (twice the
 // shared-memory words); rows without cached d and rd half as much again; the
 // hand-over between CTAs 1500.  So a grid of few rows runs in one CTA without any
 // hand-over: 12x10x8 takes 2.0 us a sweep (FP32) and 2.3 us (FP64) there against
-// 3.2 and 3.0 on 4 CTAs.
+// 3.2 and 3.0 on 4 CTAs.  These are fits of measured sweeps (the time of a step of 88 sweeps less one
+// of 24, over 64) on one B200 at its 1.9 GHz: another clock scales all of them alike and changes no
+// choice but that against the marching kernel; a change of the kernel's inner loops asks for new ones.
+//
+// Wide rows (more than 64 cells per colour): by rows, or by chunks (kResLong) where that takes at
+// most half the turns.  A ring of more cells than the threads poll at once costs 900 for each
+// further round where no interior rows cover it (200x64x64 FP32 in bricks of 2x16 rows 8.1 us, of
+// 3x11 6.8).  Bricks of one row where nothing thicker fits the chip (1572x6x3 FP64: 7.0 us a
+// sweep, by half-sweep kernels 12.3), or where the thicker ones' ring is that large and the
+// estimate at least a tenth lower (800x9x9 FP64 5.7 us against 11.8, FP32 4.0 against 8.6).
 //
 // k_sor_deep, with one hand-over a sweep, has a cost of its own: 880 (FP64 950) for the
 // hand-over and the barriers, 187 (235) per turn of the warps over the rows of a colour,
@@ -436,9 +448,8 @@ struct ResidentArgs {
 // against 3.8, 64x96x96 3.75 against 4.9) and leaves larger FP64 bricks (40x100x100: 6.3 against
 // 6.0) and those whose extra arrays do not fit.
 //
-// *us receives the time of a sweep by that estimate at 680
-// clocks a microsecond (the measured times of 17 FP32 grids of 0.3 to 3.1 M cells lie
-// within 10% of it where d is cached; rows of less than 32 pairs take up to 1.6
+// *us receives the time of a sweep by that estimate (the measured times of 17 FP32 grids of 0.3 to
+// 3.1 M cells lie within 10% of it where d is cached; rows of less than 32 pairs take up to 1.6
 // times the estimate, wide ones 1.1).  Returns false when no plan fits one CTA per SM.
 template <class Tc>
 bool plan_resident(ntcfd_ctx* ctx, double* us) {
@@ -447,44 +458,63 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
     const size_t limit = ctx->smem_optin > 4096 ? ctx->smem_optin - 4096 : 0;
     const int mode = res_mode(g.nx);
     const long long per = kResNT / 32 * (mode == kResNarrow ? 2 * (32 / half) : 1);   // rows of a pass
-    const double pass = (mode == kResNarrow ? 640.0 : 360.0 * ((half + 63) / 64)) * (sizeof(Tc) == 8 ? 1.7 : 1.0);
+    const int nch = (half + 63) / 64;                                                 // chunks of a row
+    const double pass = (mode == kResNarrow ? 640.0 : 360.0) * (sizeof(Tc) == 8 ? 1.7 : 1.0);
     double best = -1.0;
     Brick bb{}, db{};
     size_t bsm = 0;
     double deep = -1.0;
-    for (int nbk = 1; nbk <= std::max(1, g.nz / 2) && nbk <= ctx->sm_count; ++nbk) {
-        const int KB = (g.nz + nbk - 1) / nbk;
-        for (int nbj = 1; nbj <= std::max(1, g.ny / 2) && nbj * nbk <= ctx->sm_count; ++nbj) {
-            const int JB = (g.ny + nbj - 1) / nbj;
-            Brick b{nbj, nbk, JB, KB, mx, 0, 0, mode, 2 * (JB + KB) * half, 0};
-            if (resident_smem<Tc>(b, g.nx) > limit) continue;
-            // cache d, then rd, when they fit as well
-            b.cache_d = 1;
-            if (resident_smem<Tc>(b, g.nx) > limit) b.cache_d = 0;
-            b.cache_rd = 1;
-            if (resident_smem<Tc>(b, g.nx) > limit) b.cache_rd = 0;
-            const long long rows = (long long)JB * KB, ni = JB > 2 && KB > 2 ? (long long)(JB - 2) * (KB - 2) : 0;
-            const double cost = pass * (double)((ni + per - 1) / per + 1.6 * ((rows - ni + per - 1) / per)) *
-                                    (1.0 + 0.25 * (2 - b.cache_d - b.cache_rd)) +
-                                (nbj * nbk > 1 ? 1500.0 : 300.0) + 0.01 * (JB + KB);
-            if (best < 0 || cost < best) {
-                best = cost;
-                bb = b;
-                bsm = resident_smem<Tc>(b, g.nx);
-            }
-            Brick d = b;
-            d.deep = 1;
-            d.inbox = deep_inbox_rows(d) * half;
-            if (mode != kResNarrow || nbj * nbk < 2 || deep_smem<Tc>(d) > limit) continue;
-            const long long turn = per / 2, red = rows + 2 * ((nbj > 1 ? KB : 0) + (nbk > 1 ? JB : 0));
-            const double turns = (double)((red + turn - 1) / turn + (rows + turn - 1) / turn);
-            const double dcost = sizeof(Tc) == 8 ? 950.0 + 235.0 * turns : 880.0 + 187.0 * turns;
-            if (deep < 0 || dcost < deep) {
-                deep = dcost;
-                db = d;
+    // the edge rows' places may take of what the limit leaves
+    auto fits = [&](const Brick& b) {
+        const size_t all = resident_smem<Tc>(b, g.nx);
+        return all - resident_places(b) <= limit && all <= limit + 3072;
+    };
+    auto ring_cells = [&](const Brick& b) { return ((b.nbj > 1 ? 2 * b.KB : 0) + (b.nbk > 1 ? 2 * b.JB : 0)) * half; };
+    // (rows * chunks + per - 1) / per: turns of the warps
+    auto turns = [&](long long rows, long long chunks) { return (double)((rows * chunks + per - 1) / per); };
+    auto search = [&](bool thin) {
+        const int mostj = std::max(1, thin ? g.ny : g.ny / 2), mostk = std::max(1, thin ? g.nz : g.nz / 2);
+        for (int nbk = 1; nbk <= mostk && nbk <= ctx->sm_count; ++nbk) {
+            const int KB = (g.nz + nbk - 1) / nbk;
+            for (int nbj = 1; nbj <= mostj && nbj * nbk <= ctx->sm_count; ++nbj) {
+                if (thin && 2 * nbj <= g.ny && 2 * nbk <= g.nz) continue;
+                const int JB = (g.ny + nbj - 1) / nbj;
+                const long long rows = (long long)JB * KB, ne = res_edge_rows(JB, KB);
+                // by chunks where that takes at most half the turns
+                const double by_rows = nch * (turns(rows - ne, 1) + 1.6 * turns(ne, 1));
+                const double by_chunks = turns(rows - ne, nch) + 1.6 * turns(ne, nch);
+                const bool chunks = mode == kResWide && (thin || by_chunks <= 0.5 * by_rows);
+                Brick b{nbj, nbk, JB, KB, mx, 0, 0, chunks ? (int)kResLong : mode, 2 * (JB + KB) * half, 0};
+                if (!fits(b)) continue;
+                // cache d, then rd, when they fit as well
+                b.cache_d = 1;
+                if (!fits(b)) b.cache_d = 0;
+                b.cache_rd = 1;
+                if (!fits(b)) b.cache_rd = 0;
+                const double rounds = mode == kResWide && ne == rows ? (double)((ring_cells(b) - 1) / (kResNT * kFillOf<Tc>)) : 0.0;
+                const double cost = pass * (chunks ? by_chunks : by_rows) * (1.0 + 0.25 * (2 - b.cache_d - b.cache_rd)) +
+                                    (nbj * nbk > 1 ? 1500.0 + 900.0 * rounds : 300.0) + 0.01 * (JB + KB);
+                if (best < 0 || cost < (thin ? 0.9 : 1.0) * best) {
+                    best = cost;
+                    bb = b;
+                    bsm = resident_smem<Tc>(b, g.nx);
+                }
+                Brick d = b;
+                d.deep = 1;
+                d.inbox = deep_inbox_rows(d) * half;
+                if (mode != kResNarrow || nbj * nbk < 2 || deep_smem<Tc>(d) > limit) continue;
+                const long long red = rows + 2 * ((nbj > 1 ? KB : 0) + (nbk > 1 ? JB : 0));
+                const double dturns = turns(red, 2) + turns(rows, 2);       // one row a lane group, not two
+                const double dcost = sizeof(Tc) == 8 ? 950.0 + 235.0 * dturns : 880.0 + 187.0 * dturns;
+                if (deep < 0 || dcost < deep) {
+                    deep = dcost;
+                    db = d;
+                }
             }
         }
-    }
+    };
+    search(false);
+    if (mode == kResWide && (best < 0 || ring_cells(bb) > kResNT * (sizeof(Tc) == 4 ? 4 : 3))) search(true);
     if (deep >= 0 && deep < (sizeof(Tc) == 8 ? 0.76 : 0.85) * best) {
         best = deep;
         bb = db;
