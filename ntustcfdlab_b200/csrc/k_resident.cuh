@@ -105,9 +105,11 @@ inline size_t resident_smem(const Brick& b, int nx) {
            resident_places(b) + 64 * sizeof(Tc);
 }
 
-// ring words a thread holds in flight
+// ring words a thread holds in flight (FP64: of three many a brick's ring takes a second round of
+// polls, 101x89x105 7.7 us a sweep against 6.8; more than these in FP32 lengthen every round, 256x24x24 3.3
+// us a sweep, 4.2 with twelve)
 template <class Tc>
-constexpr int kFillOf = 24 / (int)sizeof(Tc);
+constexpr int kFillOf = sizeof(Tc) == 4 ? 6 : 4;
 
 constexpr unsigned int kNanFlag = 1u << 20;   // high-half flag of a CTA whose max |change| was not finite
 
@@ -250,6 +252,11 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     Places* const pubT = reinterpret_cast<Places*>(rowC + 4 * JB * KB);
     int2* const ringT = reinterpret_cast<int2*>(pubT + res_edge_rows(JB, KB));
     constexpr int NWARP = NT / 32;
+    // an update of its own for each parity of a row (the warp's rows have one each): without the selects by
+    // parity narrow rows take 11.3 us a sweep against 12.6 (48x192x187 FP32), 12.0 against 13.2
+    // (33x134x264 FP64), 128^3 FP64 11.2 against 11.4; other wide rows are slower so (112^3 FP64 8.7
+    // against 8.4, FP32 6.9 against 6.7)
+    constexpr bool kParity = MODE == kResNarrow || (MODE == kResWide1 && sizeof(Tc) == 8 && !CD);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tid = threadIdx.x;
 
@@ -349,7 +356,11 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
     __syncthreads();
     // the lane's cell t in the narrow form, and its row among the rpw side by side
     const int rpw = MODE == kResNarrow ? 32 / nown1 : 1;
-    const int sub = MODE == kResNarrow ? lane / nown1 : 0, lt = lane - sub * nown1;
+    // (in FP64 the lanes left over go on past the end of the last row: from a row's start they would
+    // meet the other lanes' banks)
+    const int most = sizeof(Tc) == 8 ? rpw - 1 : rpw;
+    const int sub = MODE == kResNarrow ? min(lane / nown1, most) : 0, lt = lane - sub * nown1;
+    const bool lane_in = sub < rpw && lt < nown1;
     // lane coefficients of the one- and two-row instances: the cells t = lt (and
     // t = lt + 32) of a row of parity r sit at i = 2t + 2 - r (past the row's end
     // they read other table entries, never used)
@@ -580,32 +591,53 @@ k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const d
         if constexpr (MODE == kResNarrow) {
             // rows of at most 32 cells per colour: a warp takes 2 rpw rows at a time, rpw side by
             // side over the lanes (rpw = 32 / nown1), twice
-            for (int er = e0r + 2 * rpw * warp + sub; er < e1r + sub; er += 2 * rpw * NWARP) {
-                const int eB = er + rpw;
-                const bool inA = sub < rpw && er < e1r, inB = sub < rpw && eB < e1r;
-                const ResRow<Tc> wA = row_of(inA ? er : e0r), wB = row_of(inB ? eB : e0r);
-                const int rA = (wA.par ^ c) & 1, rB = (wB.par ^ c) & 1;
+            auto pair = [&](const ResRow<Tc>& wA, const ResRow<Tc>& wB, int rA, int rB, bool inA, bool inB) __attribute__((always_inline)) {
                 const int mA = lt + 2 - rA, mB = lt + 2 - rB;
                 const ResIn<Tc> xA = res_load<Tc, CD, CR>(wA, lt, mA, mx, plane);
                 const ResIn<Tc> xB = res_load<Tc, CD, CR>(wB, lt, mB, mx, plane);
-                res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xA, wA, lt, mA, rA ? cEr[1][0] : cEr[0][0], rA ? cWr[1][0] : cWr[0][0], om,
+                res_finish<Tc, EDGE, CD && !CR, false>(xA, wA, lt, mA, rA ? cEr[1][0] : cEr[0][0], rA ? cWr[1][0] : cWr[0][0], om,
                                      inA && lt < (rA ? nown1 : nown0), inA, seq, ch);
-                res_finish<Tc, EDGE, CD && !CR, MODE == kResLong>(xB, wB, lt, mB, rB ? cEr[1][0] : cEr[0][0], rB ? cWr[1][0] : cWr[0][0], om,
+                res_finish<Tc, EDGE, CD && !CR, false>(xB, wB, lt, mB, rB ? cEr[1][0] : cEr[0][0], rB ? cWr[1][0] : cWr[0][0], om,
                                      inB && lt < (rB ? nown1 : nown0), inB, seq, ch);
+            };
+            if (rpw == 1) {
+                for (int er = e0r + 2 * warp; er < e1r; er += 2 * NWARP) {
+                    const bool inB = lane_in && er + 1 < e1r;
+                    const ResRow<Tc> wA = row_of(er), wB = row_of(er + 1 < e1r ? er + 1 : er);
+                    const int rA = (wA.par ^ c) & 1, rB = (wB.par ^ c) & 1;
+                    if (rA == 0) {
+                        if (rB == 0) pair(wA, wB, 0, 0, lane_in, inB);
+                        else pair(wA, wB, 0, 1, lane_in, inB);
+                    } else {
+                        if (rB == 0) pair(wA, wB, 1, 0, lane_in, inB);
+                        else pair(wA, wB, 1, 1, lane_in, inB);
+                    }
+                }
+            } else {
+                for (int er = e0r + 2 * rpw * warp + sub; er < e1r + sub; er += 2 * rpw * NWARP) {
+                    const int eB = er + rpw;
+                    const bool inA = lane_in && er < e1r, inB = lane_in && eB < e1r;
+                    const ResRow<Tc> wA = row_of(er < e1r ? er : e0r), wB = row_of(eB < e1r ? eB : e0r);
+                    pair(wA, wB, (wA.par ^ c) & 1, (wB.par ^ c) & 1, inA, inB);
+                }
             }
         } else if constexpr (MODE == kResWide1) {
             for (int er = e0r + warp; er < e1r; er += NWARP) {
                 const ResRow<Tc> w = row_of(er);
-                const int r = (w.par ^ c) & 1;
-                const int nown = r ? nown1 : nown0;
                 // cells t = lane (always in the row: it holds more than 32) and lane + 32
-                const int m = lane + 2 - r;
-                const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, lane, m, mx, plane);
-                const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, lane + 32, m + 32, mx, plane);
-                res_finish<Tc, EDGE, CD && !CR, false>(xA, w, lane, m, r ? cEr[1][0] : cEr[0][0], r ? cWr[1][0] : cWr[0][0], om, true, true,
-                                     seq, ch);
-                res_finish<Tc, EDGE, CD && !CR, false>(xB, w, lane + 32, m + 32, r ? cEr[1][1] : cEr[0][1], r ? cWr[1][1] : cWr[0][1], om,
-                                     lane + 32 < nown, lane + 32 < nown1, seq, ch);
+                auto one = [&](int r) __attribute__((always_inline)) {
+                    const int nown = r ? nown1 : nown0, m = lane + 2 - r;
+                    const ResIn<Tc> xA = res_load<Tc, CD, CR>(w, lane, m, mx, plane);
+                    const ResIn<Tc> xB = res_load<Tc, CD, CR>(w, lane + 32, m + 32, mx, plane);
+                    res_finish<Tc, EDGE, CD && !CR, false>(xA, w, lane, m, r ? cEr[1][0] : cEr[0][0], r ? cWr[1][0] : cWr[0][0], om, true,
+                                         true, seq, ch);
+                    res_finish<Tc, EDGE, CD && !CR, false>(xB, w, lane + 32, m + 32, r ? cEr[1][1] : cEr[0][1], r ? cWr[1][1] : cWr[0][1],
+                                         om, lane + 32 < nown, lane + 32 < nown1, seq, ch);
+                };
+                const int r = (w.par ^ c) & 1;
+                if (kParity && r) one(1);
+                else if (kParity) one(0);
+                else one(r);
             }
         } else {
             // the cells t0 + lane, and with `two` t0 + 32 + lane, of a row

@@ -55,7 +55,7 @@ k_sor_deep(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const Tc* _
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using B = decltype(abs_bits(Tc(0)));
     using Word = RingWord<Tc>;
-    constexpr int NWARP = NT / 32, kFill = kFillOf<Tc>;
+    constexpr int NWARP = NT / 32, kFill = 24 / (int)sizeof(Tc);   // ring words a thread holds in flight
     __shared__ int s_flag, s_fail[2], s_nan[2];
     __shared__ uint2 s_vd;                        // this sweep's red verdicts, the last sweep's black ones
     __shared__ unsigned int s_prev[2][4];
