@@ -91,8 +91,9 @@ struct ntcfd_ctx {
     double *us = nullptr, *vs = nullptr, *ws = nullptr, *b = nullptr;
     double *eta = nullptr, *nut = nullptr;
     double* fb = nullptr;                   // body force fu, fv, fw (3 natural arrays), null when unset
+    // e, d and 1/diag (sweep precision) per colour; made when first needed (split_arrays)
     void *eR = nullptr, *eB = nullptr, *dR = nullptr, *dB = nullptr;
-    void *rdR = nullptr, *rdB = nullptr;   // 1/diag per colour (sweep precision)
+    void *rdR = nullptr, *rdB = nullptr;
     double* tabd = nullptr;   // double tables
     float* tabf = nullptr;    // float tables
     Tabs<double> tpd{};
@@ -119,8 +120,10 @@ struct ntcfd_ctx {
     unsigned long long* boxes = nullptr;    // its inboxes (made with the first plan, kept)
     size_t box_words = 0;
     Brick brick{};
-    bool resident = false;                  // the graph uses the resident SOR kernel
-    bool march = false;                     // the graph uses the marching SOR kernel
+    // the pressure solve's kernel, chosen when the context is made (choose_solve)
+    bool resident = false;                  // the resident SOR kernel
+    bool march = false;                     // the marching SOR kernel
+    bool solve_ready = false;               // it is in use (ready_solve)
     MarchPlan mplan{};
     void* mf = nullptr;                     // its e (two buffers) and d
     size_t res_smem = 0;
@@ -615,55 +618,87 @@ bool plan_march(ntcfd_ctx* ctx, MarchPlan* plan, double* us) {
     return best >= 0;
 }
 
-// Takes the plan into use: the kernel's attributes and its arrays (kept with the
-// context; not when they would take a quarter of the free memory).
+// Takes the plan into use: the kernel's attributes.
 template <class Tc>
-bool use_march(ntcfd_ctx* ctx, const MarchPlan& m) {
+bool use_march(ntcfd_ctx* ctx) {
+    const MarchPlan& m = ctx->mplan;
     int per_sm = 0;
-    size_t free_b = 0, total = 0;
     const void* kern = march_kernel<Tc>(m.HP);
     if (!allow_smem(ctx, kern, m.smem) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, m.nt, m.smem) != cudaSuccess ||
-        (long long)m.nbj * m.nbk > (long long)per_sm * ctx->sm_count ||
-        (!ctx->mf && cudaMemGetInfo(&free_b, &total) != cudaSuccess)) {
+        (long long)m.nbj * m.nbk > (long long)per_sm * ctx->sm_count) {
         cudaGetLastError();
         return false;
     }
-    if (!ctx->mf) {
-        Tc* q;
-        if (6 * m.elems * sizeof(Tc) > free_b / 4 || dalloc(ctx, &q, 6 * m.elems)) {
-            cudaGetLastError();
-            return false;
-        }
-        ctx->mf = q;
-    }
-    ctx->mplan = m;
     return true;
 }
 
-// Chooses the kernels of the pressure solve.  The resident kernel where e fits the
+// 1/diag of the metrics, where the arrays are there.
+template <class Tc>
+int make_rd(ntcfd_ctx* ctx) {
+    if (!ctx->rdR) return 0;
+    const dim3 b3(32, 4, 2), g3 = grid3(ctx->g, b3);
+    k_make_rd<Tc><<<g3, b3, 0, ctx->stream>>>(ctx->g, sor_coef<Tc>(ctx), (Tc*)ctx->rdR, (Tc*)ctx->rdB);
+    CK(cudaGetLastError());
+    return 0;
+}
+
+// The colour-split e, d and 1/diag: made with the context unless its solves march, else
+// when a call needs them (the z-slab stages).
+template <class Tc>
+int split_arrays(ntcfd_ctx* ctx) {
+    if (ctx->eR) return 0;
+    void* a[6];
+    for (void*& q : a) {
+        Tc* t;
+        if (int rc = dalloc(ctx, &t, ctx->spl_elems)) return rc;
+        q = t;
+    }
+    ctx->eR = a[0]; ctx->eB = a[1]; ctx->dR = a[2]; ctx->dB = a[3]; ctx->rdR = a[4]; ctx->rdB = a[5];
+    return ctx->metrics_set ? make_rd<Tc>(ctx) : 0;
+}
+
+// Chooses the kernel of the pressure solve, once per context, from the grid and the device: steps and
+// adjoints of a context run in one kernel from its first to its last.  The resident kernel where e fits the
 // chip, except in FP32 where the marching kernel is estimated 5% faster: on grids too large
-// for its d on the chip (64x192x256: 14.0 us a sweep with restarts against 16.7, 140^3:
-// 13.6 against 18.0) and narrow ones (33x150x220: 9.8 against 12.9); on 15 others of 0.3 to
+// for its d on the chip (64x192x256: 13.8 us a sweep with restarts against 14.4, 140^3:
+// 13.5 against 15.9) and narrow ones (33x150x220: 9.8 against 10.9); on 15 others of 0.3 to
 // 2 M cells the resident kernel takes 5.2 to 12.9 us against 7.5 to 13.4.  FP64 sweeps
-// march slower (128^3: 15.5 us against 11.3).  Then the marching kernel where it has a plan, else
-// two kernels a sweep.
+// march slower (128^3: 15.7 us against 11.2).  Then the marching kernel where it has a plan, else
+// two kernels a sweep.  A marching context holds that kernel's arrays in place of the colour-split
+// ones; where they do not fit the memory it takes the next kernel.
 template <class Tc>
 int choose_solve(ntcfd_ctx* ctx) {
     const int path = ctx->prm.sor_path;
     double tr = 0.0, tm = 0.0;
-    MarchPlan mp;
-    ctx->march = ctx->resident = false;
+    if (is_slab(ctx)) return split_arrays<Tc>(ctx);   // its stages are half-sweeps
     const bool fits = path != NTCFD_SOR_STREAMING && plan_resident<Tc>(ctx, &tr);
-    if (path == NTCFD_SOR_RESIDENT) {
-        ctx->resident = fits && use_resident<Tc>(ctx);
-        if (!ctx->resident) return fail(ctx, NTCFD_EINVAL, "the resident SOR kernel does not fit this grid on this device");
-        return 0;
+    const bool marches = path != NTCFD_SOR_RESIDENT && plan_march<Tc>(ctx, &ctx->mplan, &tm);
+    ctx->resident = fits && !(marches && sizeof(Tc) == 4 && tm <= 0.95 * tr);
+    if (!ctx->resident && marches) {
+        Tc* q;
+        if (dalloc(ctx, &q, 6 * ctx->mplan.elems) == 0) {
+            ctx->mf = q;
+            ctx->march = true;
+            return 0;
+        }
+        cudaGetLastError();
+        ctx->err.clear();
+        ctx->resident = fits;
     }
-    const bool marches = plan_march<Tc>(ctx, &mp, &tm);
-    if (fits && !(marches && sizeof(Tc) == 4 && tm <= 0.95 * tr)) ctx->resident = use_resident<Tc>(ctx);
-    if (!ctx->resident && marches) ctx->march = use_march<Tc>(ctx, mp);
-    if (!ctx->resident && !ctx->march && fits) ctx->resident = use_resident<Tc>(ctx);
+    return split_arrays<Tc>(ctx);
+}
+
+// Takes the chosen kernel into use, before the first step; if the device refuses it, the
+// half-sweep kernels for good.
+template <class Tc>
+int ready_solve(ntcfd_ctx* ctx) {
+    if (ctx->solve_ready) return 0;
+    if (ctx->resident && !use_resident<Tc>(ctx)) ctx->resident = false;
+    if (ctx->march && !use_march<Tc>(ctx)) ctx->march = false;
+    if (!ctx->march)
+        if (int rc = split_arrays<Tc>(ctx)) return rc;
+    ctx->solve_ready = true;
     return 0;
 }
 
@@ -736,7 +771,9 @@ int add_step_nodes(ntcfd_ctx* ctx, cudaGraph_t G, int extra) {
                   (const double*)ctx->v, (const double*)ctx->w, (const double*)ctx->us,
                   (const double*)ctx->vs, (const double*)ctx->ws, ctx->b, P.dt, back_iface(ctx)));
     dep = {n};
-    if (int rc = choose_solve<Tc>(ctx)) return rc;
+    if (int rc = ready_solve<Tc>(ctx)) return rc;
+    if (P.sor_path == NTCFD_SOR_RESIDENT && !ctx->resident)
+        return fail(ctx, NTCFD_EINVAL, "the resident SOR kernel does not fit this grid on this device");
     if (ctx->resident) {
         // the resident kernel runs the whole solve (every correction cycle), so the
         // solve is two plain nodes: the defect (which also starts the solve) and the kernel
@@ -1132,10 +1169,11 @@ int time_kernels_t(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
                                                ctx->ws, ctx->b, P.dt, back_iface(ctx));
          }, &out->rhs_ms, 1)))
         return rc;
+    if ((rc = ready_solve<Tc>(ctx))) return rc;
     Tc *eR = (Tc*)ctx->eR, *eB = (Tc*)ctx->eB, *dR = (Tc*)ctx->dR, *dB = (Tc*)ctx->dB;
     // the defect the path's restarts use: k_defect (resident), k_defect_rows (streaming;
     // the marching kernel's below)
-    if ((rc = timed([&] {
+    if (!ctx->march && (rc = timed([&] {
              if (ctx->resident)
                  k_defect<Tc><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, ctx->p, ctx->b, dR, dB, eR, eB,
                                                           (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, 0, 0,
@@ -1296,13 +1334,6 @@ int ntcfd_create(const ntcfd_params* prm, ntcfd_ctx** out) {
     for (double** a : nat)
         if ((rc = dalloc(ctx, a, N))) return rc;
     if (P.LES && (rc = dalloc(ctx, &ctx->nut, N))) return rc;
-    const size_t esz = P.precision == NTCFD_MIXED ? sizeof(float) : sizeof(double);
-    void** spl[] = {&ctx->eR, &ctx->eB, &ctx->dR, &ctx->dB, &ctx->rdR, &ctx->rdB};
-    for (void** a : spl) {
-        char* q;
-        if ((rc = dalloc(ctx, &q, ctx->spl_elems * esz))) return rc;
-        *a = q;
-    }
     ctx->nchunk = (P.nz + kProjKc - 1) / kProjKc;
     const size_t cols = (size_t)P.nx * P.ny;
     if ((rc = dalloc(ctx, &ctx->partZ, cols * ctx->nchunk))) return rc;
@@ -1348,6 +1379,7 @@ int ntcfd_create(const ntcfd_params* prm, ntcfd_ctx** out) {
     ctx->coordY = ctx->coordbuf + 1;                  // Y[j] valid for j = -1..ny+3
     ctx->coordZ = ctx->coordbuf + (P.ny + 5) + 4 + 1;
     if (ctx->csweeps > 64) return fail(ctx, NTCFD_EINVAL, "check_every must be <= 64");
+    if ((rc = P.precision == NTCFD_MIXED ? choose_solve<float>(ctx) : choose_solve<double>(ctx))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     return 0;
 }
@@ -1448,14 +1480,7 @@ int ntcfd_set_metrics(ntcfd_ctx* ctx, const double* iDx, const double* Dxs, cons
         ctx->tpd.ax[ax] = AxisTabs<double>{tb, tb + Lx, tb + 2 * Lx, tb + 3 * Lx, tb + 4 * Lx, tb + 5 * Lx};
         ctx->tpf.ax[ax] = AxisTabs<float>{tf, tf + Lx, tf + 2 * Lx, tf + 3 * Lx, tf + 4 * Lx, tf + 5 * Lx};
     }
-    {
-        const dim3 b3(32, 4, 2), g3 = grid3(g, b3);
-        if (ctx->prm.precision == NTCFD_MIXED)
-            k_make_rd<float><<<g3, b3, 0, ctx->stream>>>(g, ctx->scf, (float*)ctx->rdR, (float*)ctx->rdB);
-        else
-            k_make_rd<double><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, (double*)ctx->rdR, (double*)ctx->rdB);
-        CK(cudaGetLastError());
-    }
+    if (int rc = ctx->prm.precision == NTCFD_MIXED ? make_rd<float>(ctx) : make_rd<double>(ctx)) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->metrics_set = true;
     drop_graphs(ctx);
@@ -1896,9 +1921,10 @@ long long ntcfd_slab_plane_elems(const ntcfd_ctx* ctx, int field) {
 int ntcfd_slab_planes(ntcfd_ctx* ctx, int field, int k0, int count, double* buf, int put) {
     DEV();
     long long plane = 0;
-    double* f = slab_field(ctx, field, &plane);
-    if (!f) return fail(ctx, NTCFD_EINVAL, "unknown field %d", field);
+    if (field < NTCFD_FIELD_U || field > NTCFD_FIELD_E_BLACK) return fail(ctx, NTCFD_EINVAL, "unknown field %d", field);
     if (ctx->prm.precision != NTCFD_FP64) return fail(ctx, NTCFD_EINVAL, "the z-slab stages run in FP64");
+    if (int rc = split_arrays<double>(ctx)) return rc;
+    double* f = slab_field(ctx, field, &plane);
     if (!buf || count < 1 || k0 < -1 || k0 + count - 1 > ctx->g.nz + 2)
         return fail(ctx, NTCFD_EINVAL, "planes %d..%d outside -1..nz+2", k0, k0 + count - 1);
     double* dev = f + plane * (long long)(k0 + 1);
@@ -1913,6 +1939,7 @@ int ntcfd_slab_stage(ntcfd_ctx* ctx, int stage, int colour) {
     DEV();
     if (!ctx->metrics_set) return fail(ctx, NTCFD_ESTATE, "ntcfd_set_metrics must come first");
     if (ctx->prm.precision != NTCFD_FP64) return fail(ctx, NTCFD_EINVAL, "the z-slab stages run in FP64");
+    if (int rc = split_arrays<double>(ctx)) return rc;
     const Geom g = ctx->g;
     const ntcfd_params& P = ctx->prm;
     cudaStream_t st = ctx->stream;
