@@ -273,8 +273,9 @@ def cpu_baseline_from(s_gpu, case, seconds, threads=None):
 
 def roofline(s, case, path, reps=20):
     """Dominant kernel: the SOR sweeps.  Algorithmic bytes: 3 S per cell per
-    full red+black sweep (read e, d and rd, write e of every cell once; S = 4 B
-    mixed, 8 B FP64).  Streaming path: one launch = one colour = 1.5 S per
+    full red+black sweep (read e and d, write e of every cell once; S = 4 B
+    mixed, 8 B FP64).  Streaming path: half of a sweep (a launch of one colour, or half of a
+    sweep of the marching kernel) = 1.5 S per
     cell.  Resident path: one launch runs `resident_sweeps` sweeps (timed
     standalone, zeta = 0).
 
@@ -288,15 +289,18 @@ def roofline(s, case, path, reps=20):
 
     `per_kernel` gives each stencil kernel's algorithmic bytes per launch
     over its CUDA-event time as a fraction of the measured HBM bandwidth."""
+    from ntustcfdlab_b200 import abi
     kt = s.time_kernels(reps)
     S = 4 if case.params.precision == 1 else 8
     N = case.cells
     if path == 2 and kt["resident_ms"] > 0:
-        kernel = "k_sor_resident (all sweeps of a correction cycle, e in shared memory)"
+        deep = s.solve_plan()["kernel"] == abi.SOLVE_RESIDENT_DEEP
+        kernel = f"{'k_sor_deep' if deep else 'k_sor_resident'} (all sweeps of a solve, e in shared memory)"
         alg = 3 * S * N * kt["resident_sweeps"]
         ms = kt["resident_ms"]
     else:
-        kernel = "k_sor_march, or k_sweep of wide rows (half a red-black SOR sweep)"
+        kernel = {abi.SOLVE_MARCH: "k_sor_march (half of a sweep: the sweeps of a solve in one launch)",
+                  abi.SOLVE_HALF_SWEEPS: "k_sweep (one colour of a red-black SOR sweep)"}[s.solve_plan()["kernel"]]
         alg = 1.5 * S * N
         ms = kt["sweep_ms"]
     ach = alg / (ms * 1e-3) / 1e9

@@ -205,6 +205,12 @@ module ntcfd_iface
          type(ntcfd_kernel_times), intent(out) :: times
       end function
 
+      integer(c_int) function ntcfd_solve_plan(ctx, plan) bind(C, name="ntcfd_solve_plan")
+         import :: c_int, c_ptr
+         type(c_ptr), value :: ctx
+         integer(c_int), intent(out) :: plan(5)
+      end function
+
       integer(c_int) function ntcfd_set_dynamic_aoa(ctx, az, ay, npts, aoa1, reduce_frequency, zc, yc, &
             start_step) bind(C, name="ntcfd_set_dynamic_aoa")
          import :: c_int, c_ptr, c_double

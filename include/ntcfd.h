@@ -71,6 +71,9 @@ enum { NTCFD_SOR_REDBLACK = 0, NTCFD_SOR_LEX = 1 };    /* LEX: oracle only */
  * AUTO      -- RESIDENT when it fits and is the faster, else STREAMING.  All
  *              run the same red-black iteration and stop rule. */
 enum { NTCFD_SOR_AUTO = 0, NTCFD_SOR_STREAMING = 1, NTCFD_SOR_RESIDENT = 2 };
+/* The kernel of a context's pressure solves (ntcfd_solve_plan): half-sweeps and marching are
+ * the STREAMING path, the other two the RESIDENT one (DEEP: a two-row ring, one hand-over a sweep). */
+enum { NTCFD_SOLVE_HALF_SWEEPS = 0, NTCFD_SOLVE_MARCH = 1, NTCFD_SOLVE_RESIDENT = 2, NTCFD_SOLVE_RESIDENT_DEEP = 3 };
 
 typedef struct ntcfd_params {
     int nx, ny, nz;          /* interior cells (variables_module.f90:13-17) */
@@ -231,6 +234,11 @@ int ntcfd_last_step_ms(const ntcfd_ctx* ctx, float* ms);
  * stream with CUDA events and returns the averages.  The velocity, pressure
  * and ETA of the context are left unchanged. */
 int ntcfd_time_kernels(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out);
+
+/* The pressure solve chosen for the context: plan[0] the kernel (NTCFD_SOLVE_*), plan[1] and
+ * plan[2] its tiles along j and k (one CTA each; 0 for half-sweeps), plan[3] and plan[4] whether
+ * the defect and 1/diag are kept in shared memory. */
+int ntcfd_solve_plan(const ntcfd_ctx* ctx, int plan[5]);
 
 /* dynamic_AOA + RayCasting inside the time loop (airfoil.f90:311-321,
  * main.f90:144-155).  From the context's step start_step on (steps counted

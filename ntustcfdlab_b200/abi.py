@@ -32,6 +32,7 @@ QUICK_CENTRE, QUICK, UPWIND, CENTRE = 0, 1, 2, 3   # K2 schemes (discretisation_
 SMAG_REF_ALIASED, SMAG_STAGGERED = 0, 1
 SOR_REDBLACK, SOR_LEX = 0, 1
 SOR_AUTO, SOR_STREAMING, SOR_RESIDENT = 0, 1, 2
+SOLVE_HALF_SWEEPS, SOLVE_MARCH, SOLVE_RESIDENT, SOLVE_RESIDENT_DEEP = range(4)   # ntcfd_solve_plan
 
 # boundary-condition strings of variables_module.f90:110-132
 BC_NAMES = {"no-slip": BC_NOSLIP, "Neumann": BC_NEUMANN, "Dirichlet": BC_DIRICHLET,
@@ -183,6 +184,7 @@ SIGNATURES = {
     "ntcfd_last_step_ms": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_float)]),
     "ntcfd_time_kernels": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int,
                                           ctypes.POINTER(NtcfdKernelTimes)]),
+    "ntcfd_solve_plan": (ctypes.c_int, [ctypes.c_void_p, _IP]),
     "ntcfd_set_body_force": (ctypes.c_int, [ctypes.c_void_p] + [_DP] * 3),
     "ntcfd_set_dynamic_aoa": (ctypes.c_int, [ctypes.c_void_p, _DP, _DP, ctypes.c_int] + [ctypes.c_double] * 4
                               + [ctypes.c_int]),

@@ -2114,6 +2114,16 @@ int ntcfd_time_kernels(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
                                             : time_kernels_t<double>(ctx, reps, out);
 }
 
+int ntcfd_solve_plan(const ntcfd_ctx* ctx, int plan[5]) {
+    if (!ctx || !ctx->stream || !plan) return NTCFD_EINVAL;
+    const Brick& b = ctx->brick;
+    const int none[5] = {NTCFD_SOLVE_HALF_SWEEPS, 0, 0, 0, 0};
+    const int march[5] = {NTCFD_SOLVE_MARCH, ctx->mplan.nbj, ctx->mplan.nbk, 0, 0};
+    const int chip[5] = {b.deep ? NTCFD_SOLVE_RESIDENT_DEEP : NTCFD_SOLVE_RESIDENT, b.nbj, b.nbk, b.cache_d, b.cache_rd};
+    std::memcpy(plan, ctx->resident ? chip : ctx->march ? march : none, sizeof none);
+    return 0;
+}
+
 // ------------------------------------------------------------------ masks
 int ntcfd_build_mask_cylinder(ntcfd_ctx* ctx, double zc, double yc, double r) {
     DEV();

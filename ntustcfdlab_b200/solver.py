@@ -273,6 +273,12 @@ class Solver:
         self._check(self.lib.ntcfd_last_step_ms(self.h, ctypes.byref(ms)))
         return ms.value
 
+    def solve_plan(self) -> dict:
+        """The pressure solve's kernel (abi.SOLVE_*), its tiles along j and k and what it keeps on the chip."""
+        plan = (ctypes.c_int * 5)()
+        self._check(self.lib.ntcfd_solve_plan(self.h, plan))
+        return dict(zip(("kernel", "nbj", "nbk", "d_cached", "rd_cached"), plan))
+
     def time_kernels(self, reps: int = 20) -> dict:
         """Average device time (ms) of standalone launches of the step kernels."""
         t = abi.NtcfdKernelTimes()
