@@ -249,7 +249,7 @@ __device__ __forceinline__ Rows<double> fma_rn(Rows<double> a, Rows<double> b, R
 __device__ __forceinline__ Rows<double> add_rn(Rows<double> a, Rows<double> b) { return {a.v + b.v}; }
 __device__ __forceinline__ Rows<double> sub_rn(Rows<double> a, Rows<double> b) { return {sub_rn(a.v, b.v)}; }
 
-// 1 / diag of the coefficient sum s, with the coefficients' sign (rdiag32, two rows at once).
+// 1 / diag of the coefficient sum s, with the coefficients' sign (rdiag_near, two rows at once).
 __device__ __forceinline__ Rows<float> march_rd(Rows<float> s) {
     float a, b;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(-s.get(0)));
@@ -257,7 +257,7 @@ __device__ __forceinline__ Rows<float> march_rd(Rows<float> s) {
     const Rows<float> x = Rows<float>::of(a, b);
     return fma_rn(x, fma_rn(s, x, Rows<float>::of(1.0f, 1.0f)), x);
 }
-__device__ __forceinline__ Rows<double> march_rd(Rows<double> s) { return {rdiag64(s.v)}; }
+__device__ __forceinline__ Rows<double> march_rd(Rows<double> s) { return {rdiag_near(s.v)}; }
 
 // Barriers in shared memory (mbarrier) and the bulk copies that complete on them.
 __device__ __forceinline__ unsigned int sm32(const void* p) { return (unsigned int)__cvta_generic_to_shared(p); }

@@ -76,15 +76,25 @@ __device__ __forceinline__ double rdiag64(double s) {
     return x;
 }
 
-// FP32, to nearest for a normal sum with a normal reciprocal: the hardware's approximation
-// and one Newton-Raphson step, whose remainder the FMA keeps exactly.
-__device__ __forceinline__ float rdiag32(float s) {
+// 1 / s to nearest, as rcp_rn gives it, for a normal sum with a normal reciprocal: the kernels that
+// form 1/diag in a sweep take the same values as those that read it (make_rd).  The hardware's
+// approximation, then steps whose remainder 1 - s x the FMA keeps exactly; the last one rounds to
+// nearest when x is within an ulp (Markstein, IBM J. Res. Dev. 34, 1990).  FP32: one step (equal to
+// rcp_rn for every significand).  FP64: a third-order step to within an ulp, rounded up, since the
+// last step ties for a significand of ones only if it comes from below; then the last (equal for 10^11
+// random sums, of which two Newton-Raphson steps miss 14 to 20).
+__device__ __forceinline__ float rdiag_near(float s) {
     float x;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(s));
     return fma_rn(x, fma_rn(-s, x, 1.0f), x);
 }
-__device__ __forceinline__ float rdiag_near(float s) { return rdiag32(s); }
-__device__ __forceinline__ double rdiag_near(double s) { return rdiag64(s); }
+__device__ __forceinline__ double rdiag_near(double s) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(s));
+    const double r = fma_rn(-s, x, 1.0);
+    x = __fma_ru(x, fma_rn(r, r, r), x);
+    return fma_rn(x, fma_rn(-s, x, 1.0), x);
+}
 
 // The FP64 defect of p + e from the defect d of p and the correction e of a
 // defect-correction cycle: since the operator is linear,
