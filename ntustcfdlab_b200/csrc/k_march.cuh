@@ -739,7 +739,8 @@ __global__ void __launch_bounds__(kMarchNT + 32, 1) k_sor_march(const __grid_con
             const unsigned int over = s_over;
             chs = cb;
             done_c = s + 1;
-            if (a.check_every == 1 || ik >= a.itmax || ik % a.check_every == 0) {
+            // every check_every sweeps of the cycle and at its end, as the half-sweep loops test
+            if (a.check_every == 1 || ik >= a.itmax || s + 1 >= a.cycle_len || (s + 1) % a.check_every == 0) {
                 tested = true;
                 nonfinite = over >= (1u << 20);
                 conv = over == 0u;
