@@ -206,7 +206,7 @@ __device__ __forceinline__ void res_finish(const ResIn<Tc>& x, const ResRow<Tc>&
 
 template <class Tc, int NT, bool CD, bool CR, int MODE>
 __global__ void __launch_bounds__(NT, 1)
-k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p, const double* __restrict__ b,
+k_sor_resident(Geom g, SorCoef<Tc> sc, Brick br, double* __restrict__ p,
                Tc* __restrict__ dRg, Tc* __restrict__ dBg, const Tc* __restrict__ rdRg,
                const Tc* __restrict__ rdBg, Ctl* ctl, ResSync* sync, unsigned long long* boxes,
                double omega, double zeta, int itmax, int cycle_len, int check_every) {

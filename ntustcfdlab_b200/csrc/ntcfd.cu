@@ -367,7 +367,7 @@ SorCoef<float> sor_coef<float>(ntcfd_ctx* ctx) { return ctx->scf; }
 
 // The resident SOR kernel for a brick plan (d and rd cached or not, row shape).
 template <class Tc>
-using ResidentFn = void (*)(Geom, SorCoef<Tc>, Brick, double*, const double*, Tc*, Tc*, const Tc*, const Tc*, Ctl*,
+using ResidentFn = void (*)(Geom, SorCoef<Tc>, Brick, double*, Tc*, Tc*, const Tc*, const Tc*, Ctl*,
                             ResSync*, unsigned long long*, double, double, int, int, int);
 template <class Tc, int MODE>
 ResidentFn<Tc> resident_kernel_m(const Brick& b) {
@@ -397,7 +397,6 @@ struct ResidentArgs {
     SorCoef<Tc> sc;
     Brick br;
     double* p;
-    const double* b;
     Tc *dR, *dB;
     const Tc *rdR, *rdB;
     Ctl* ctl;
@@ -405,17 +404,17 @@ struct ResidentArgs {
     unsigned long long* boxes;
     double omega, zeta;
     int itmax, cycle_len, check_every;
-    void* arg[17];
-    ResidentArgs(ntcfd_ctx* ctx, double* p_, const double* b_, double omega_, double zeta_, int itmax_, int cycle_,
+    void* arg[16];
+    ResidentArgs(ntcfd_ctx* ctx, double* p_, double omega_, double zeta_, int itmax_, int cycle_,
                  int check_)
-        : g(ctx->g), sc(sor_coef<Tc>(ctx)), br(ctx->brick), p(p_), b(b_), dR((Tc*)ctx->dR), dB((Tc*)ctx->dB),
+        : g(ctx->g), sc(sor_coef<Tc>(ctx)), br(ctx->brick), p(p_), dR((Tc*)ctx->dR), dB((Tc*)ctx->dB),
           rdR((const Tc*)ctx->rdR), rdB((const Tc*)ctx->rdB), ctl(ctx->ctl), sync(ctx->rsync), boxes(ctx->boxes),
           omega(omega_), zeta(zeta_), itmax(itmax_), cycle_len(cycle_), check_every(check_) {
-        void* all[] = {&g, &sc, &br, &p, &b, &dR, &dB, &rdR, &rdB, &ctl, &sync, &boxes, &omega, &zeta, &itmax, &cycle_len,
+        void* all[] = {&g, &sc, &br, &p, &dR, &dB, &rdR, &rdB, &ctl, &sync, &boxes, &omega, &zeta, &itmax, &cycle_len,
                        &check_every};
         int k = 0;
-        for (int q = 0; q < 17; ++q)
-            if (!br.deep || (q != 4 && q != 7 && q != 8)) arg[k++] = all[q];   // no b, no rd
+        for (int q = 0; q < 16; ++q)
+            if (!br.deep || (q != 6 && q != 7)) arg[k++] = all[q];   // no rd
     }
     ResidentArgs(const ResidentArgs&) = delete;
 };
@@ -782,7 +781,7 @@ int add_step_nodes(ntcfd_ctx* ctx, cudaGraph_t G, int extra) {
                       (const double*)ctx->b, dR, dB, eR, eB, (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl,
                       (cudaGraphConditionalHandle)0, 0, ctx->rsync, 1, 0));
         dep = {n};
-        ResidentArgs<Tc> ra(ctx, ctx->p, ctx->b, P.omega, P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps);
+        ResidentArgs<Tc> ra(ctx, ctx->p, P.omega, P.zeta, P.itmax, ctx->cycle_len, ctx->csweeps);
         GK(add_cooperative(&n, G, dep, resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ctx->res_smem,
                            ra.arg));
         dep = {n};
@@ -975,7 +974,7 @@ int sor_solve_eager(ntcfd_ctx* ctx, double* p, const double* b, double zeta, int
         // one defect (starting the solve) and one launch that runs every cycle
         k_defect<Tc><<<g3, b3, 0, st>>>(g, ctx->scd, p, b, dR, dB, eR, eB, (const Tc*)ctx->rdR,
                                         (const Tc*)ctx->rdB, ctx->ctl, 0, 0, ctx->rsync, 1, 0);
-        ResidentArgs<Tc> ra(ctx, p, b, omega, zeta, itmax, ctx->cycle_len, ctx->csweeps);
+        ResidentArgs<Tc> ra(ctx, p, omega, zeta, itmax, ctx->cycle_len, ctx->csweeps);
         CK(cudaLaunchCooperativeKernel(resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ra.arg,
                                        ctx->res_smem, st));
         if (int rc = read_ctl()) return rc;
@@ -1227,7 +1226,7 @@ int time_kernels_t(ntcfd_ctx* ctx, int reps, ntcfd_kernel_times* out) {
             k_defect<Tc><<<g3, b3, 0, ctx->stream>>>(g, ctx->scd, pscratch, ctx->b, dR, dB, eR, eB,
                                                      (const Tc*)ctx->rdR, (const Tc*)ctx->rdB, ctx->ctl, 0, 0,
                                                      ctx->rsync, 1, 0);
-            ResidentArgs<Tc> ra(ctx, pscratch, ctx->b, P.omega, 0.0, *sweeps, *sweeps, 1);
+            ResidentArgs<Tc> ra(ctx, pscratch, P.omega, 0.0, *sweeps, *sweeps, 1);
             cudaLaunchCooperativeKernel(resident_handle<Tc>(ctx->brick), dim3(ctx->res_grid), dim3(kResNT), ra.arg,
                                         ctx->res_smem, ctx->stream);
         };
