@@ -444,11 +444,12 @@ struct ResidentArgs {
 //
 // k_sor_deep, with one hand-over a sweep, has a cost of its own: 880 (FP64 950) for the
 // hand-over and the barriers, 187 (235) per turn of the warps over the rows of a colour,
-// fitted to sweeps of 1.6 to 7.6 us on 18 grids.  The other estimate reads 1 / 0.85 (FP32),
-// 1 / 0.76 (FP64) of the measured times of such rows, hence the factors.  So it takes the grids of
-// small bricks (12x10x8 FP64 1.6 us a sweep against 2.3, 40^3 2.6 against 3.3, 32x96x96 FP32 2.7
-// against 3.8, 64x96x96 3.75 against 4.9) and leaves larger FP64 bricks (40x100x100: 6.3 against
-// 6.0) and those whose extra arrays do not fit.
+// fitted to sweeps of 1.6 to 7.6 us on 18 grids.  The other estimate reads more of the measured
+// times of such rows than this one, hence the factors, which part 27 grids of 9 to 64 cells a row in either
+// precision within 9%.  So it takes the grids of small bricks (12x10x8 FP64 1.6 us a sweep
+// against 2.3, 40^3 2.6 against 3.4, 32x96x96 FP32 3.4 against 4.8, 64x80x90 3.9 against 4.8) and
+// leaves larger FP64 bricks (33x116x150: 8.7 against 6.8, 40x100x100: 6.3 against 5.4) and
+// those whose extra arrays do not fit.
 //
 // *us receives the time of a sweep by that estimate (the measured times of 17 FP32 grids of 0.3 to
 // 3.1 M cells lie within 10% of it where d is cached; rows of less than 32 pairs take up to 1.6
@@ -517,7 +518,7 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
     };
     search(false);
     if (mode == kResWide && (best < 0 || ring_cells(bb) > kResNT * (sizeof(Tc) == 4 ? 4 : 3))) search(true);
-    if (deep >= 0 && deep < (sizeof(Tc) == 8 ? 0.76 : 0.85) * best) {
+    if (deep >= 0 && deep < (sizeof(Tc) == 8 ? 0.72 : 0.85) * best) {
         best = deep;
         bb = db;
         bsm = deep_smem<Tc>(db);

@@ -50,7 +50,7 @@ def test_the_kernels_of_the_tests_sizes(precision):
 
 # rows side by side on a warp (two to four) and rows that leave lanes over; d and 1/diag on the chip, d
 # alone, neither
-NARROW = [(FP64, (16, 200, 200)), (FP64, (17, 200, 300)), (FP64, (33, 134, 264)), (FP64, (48, 150, 150)),
+NARROW = [(FP64, (33, 116, 150)), (FP64, (16, 200, 200)), (FP64, (17, 200, 300)), (FP64, (33, 134, 264)), (FP64, (48, 150, 150)),
           (FP64, (48, 192, 187)), (FP64, (62, 150, 170)), (MIXED, (17, 200, 300)), (MIXED, (21, 150, 150)),
           (MIXED, (40, 100, 100)), (MIXED, (47, 192, 187)), (MIXED, (63, 160, 180))]
 
