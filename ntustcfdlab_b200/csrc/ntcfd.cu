@@ -435,10 +435,11 @@ struct ResidentArgs {
 // of 24, over 64) on one B200 at its 1.9 GHz: another clock scales all of them alike and changes no
 // choice but that against the marching kernel; a change of the kernel's inner loops asks for new ones.
 //
+// A ring of more cells than the threads poll at once costs 900 for each further round where no
+// interior rows cover it (200x64x64 FP32 in bricks of 2x16 rows 8.1 us, of 3x11 6.8).
+//
 // Wide rows (more than 64 cells per colour): by rows, or by chunks (kResLong) where that takes at
-// most half the turns.  A ring of more cells than the threads poll at once costs 900 for each
-// further round where no interior rows cover it (200x64x64 FP32 in bricks of 2x16 rows 8.1 us, of
-// 3x11 6.8).  Bricks of one row where nothing thicker fits the chip (1572x6x3 FP64: 7.0 us a
+// most half the turns.  Bricks of one row where nothing thicker fits the chip (1572x6x3 FP64: 7.0 us a
 // sweep, by half-sweep kernels 12.3), or where the thicker ones' ring is that large and the
 // estimate at least a tenth lower (800x9x9 FP64 5.7 us against 11.8, FP32 4.0 against 8.6).
 //
@@ -494,7 +495,7 @@ bool plan_resident(ntcfd_ctx* ctx, double* us) {
                 if (!fits(b)) b.cache_d = 0;
                 b.cache_rd = 1;
                 if (!fits(b)) b.cache_rd = 0;
-                const double rounds = mode == kResWide && ne == rows ? (double)((ring_cells(b) - 1) / (kResNT * kFillOf<Tc>)) : 0.0;
+                const double rounds = ne == rows ? (double)((ring_cells(b) - 1) / (kResNT * kFillOf<Tc>)) : 0.0;
                 const double cost = pass * (chunks ? by_chunks : by_rows) * (1.0 + 0.25 * (2 - b.cache_d - b.cache_rd)) +
                                     (nbj * nbk > 1 ? 1500.0 + 900.0 * rounds : 300.0) + 0.01 * (JB + KB);
                 if (best < 0 || cost < (thin ? 0.9 : 1.0) * best) {
