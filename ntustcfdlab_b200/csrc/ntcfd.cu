@@ -579,8 +579,8 @@ const void* march_kernel(int HP) {
 // most one CTA per SM, of least estimated time per sweep.  A step (one plane) takes
 // about 0.36 us and 0.024 us per warp, since its chain of updates and barriers, not
 // their number, bounds it; the planes beyond the range, the start of the copies and
-// the grid barrier cost as much as 12 steps.  (128x256x384 FP32: 35.8 us by that
-// choice; other splits of 13 to 23 tiles 36.0 to 50.7 us; 64x192x256: 11.9, others up to
+// the grid barrier cost as much as 12 steps.  (128x256x384 FP32: 35.9 us by that
+// choice; other splits of 13 to 23 tiles 36.0 to 50.7 us; 64x192x256: 11.3, others up to
 // 28 us.)  Three row groups or more, so that a tile owns two thirds of the rows it
 // updates: at 231 cells a row (three groups) a sweep takes 44 us in FP32 and 55 us in
 // FP64 against 61 and 97 us of two half-sweep passes; wider rows keep those passes.
@@ -1924,7 +1924,8 @@ int ntcfd_slab_planes(ntcfd_ctx* ctx, int field, int k0, int count, double* buf,
     long long plane = 0;
     if (field < NTCFD_FIELD_U || field > NTCFD_FIELD_E_BLACK) return fail(ctx, NTCFD_EINVAL, "unknown field %d", field);
     if (ctx->prm.precision != NTCFD_FP64) return fail(ctx, NTCFD_EINVAL, "the z-slab stages run in FP64");
-    if (int rc = split_arrays<double>(ctx)) return rc;
+    if (field >= NTCFD_FIELD_E_RED)
+        if (int rc = split_arrays<double>(ctx)) return rc;
     double* f = slab_field(ctx, field, &plane);
     if (!buf || count < 1 || k0 < -1 || k0 + count - 1 > ctx->g.nz + 2)
         return fail(ctx, NTCFD_EINVAL, "planes %d..%d outside -1..nz+2", k0, k0 + count - 1);

@@ -65,7 +65,20 @@ def test_slab_stages_of_a_marching_context():
         stage(abi.STAGE_CORRECT)
         stage(abi.STAGE_PROJECT)
         for x, y in zip(a.get_state(), b.get_state()):
-            # the same sweeps; 1/diag within an ulp, four sweeps
+            # the same four sweeps, to the tolerance of two paths
             assert np.abs(x - y).max() <= 1e-12 * max(1.0, np.abs(x).max())
         b.boundary_conditions()
         b.step(1)
+
+
+def test_velocity_planes_make_no_colour_arrays():
+    with _solver(N, FP64) as s:
+        s.boundary_conditions()
+        s.step(1)
+        n = s.lib.ntcfd_slab_plane_elems(s.h, abi.FIELD_U)
+        buf = np.zeros(n)
+        before = _free()
+        s._check(s.lib.ntcfd_slab_planes(s.h, abi.FIELD_U, 1, 1, buf.ctypes.data, 0))
+        assert before - _free() < 16 << 20
+        s._check(s.lib.ntcfd_slab_planes(s.h, abi.FIELD_E_RED, 1, 1, buf.ctypes.data, 0))
+        assert before - _free() > 6 * 8 * N[0] // 2 * N[1] * N[2]
