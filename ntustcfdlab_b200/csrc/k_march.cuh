@@ -23,11 +23,11 @@
 //
 // Bound: per cell and sweep e is read and written once and d read once, 12 bytes FP32,
 // 24 FP64, against 16 and 40 of two half-sweep passes (which also read 1/diag in FP64;
-// here it is formed from the 1-D tables).  128x256x384: FP64 59.5 us a sweep (5.1 TB/s of
-// those bytes; 119.8 before, by half-sweeps), FP32 35.8 us (58.7 before), where
+// here it is formed from the 1-D tables).  128x256x384: FP64 57.5 us a sweep (5.25 TB/s of
+// those bytes; 119.8 before, by half-sweeps), FP32 35.9 us (58.7 before), where
 // the chain of a step (copies in, shared loads, two dependent updates, barrier: 0.5 to 0.8 us)
-// and its instructions bound it; a restart 87 us (85).  64x192x256: FP64 20.8 (50.1),
-// FP32 11.9 (the resident kernel: 11.9) and its restart 25 us (39).
+// bounds it, with 38% of the issue slots used; a restart 92 us (85).  64x192x256: FP64 19.7 (50.1),
+// FP32 11.3 and its restart 21 us (39).
 // What was tried: 2, 6 and 8 rows a thread (FP32 8 rows and 256 threads: 102 us, too
 // few warps; FP64 2 rows and 512: 65 us), copies 3 steps ahead (the same time), per-thread asynchronous
 // copies and one CTA barrier a step (FP64 81 us), loads into registers a step ahead

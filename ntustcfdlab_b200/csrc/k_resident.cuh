@@ -18,10 +18,11 @@
 // other colour, which its neighbour published after reading the first: no word is
 // overwritten unread.  A grid barrier per half-sweep and a copy of the published
 // rows afterwards, which this replaces, took 3.4 us of an 8.0 us FP32 sweep at 128^3.
-// A sweep takes 6.2 us at 128^3 FP32 (8.0 before), 11.4 FP64 (11.8), 3.3 us at 40^3
-// (5.3) and 3.5 us at 32x96x96 (6.2): on small grids the hand-over, some 1.5 us per
+// A sweep takes 6.4 us at 128^3 FP32 (8.0 before), 11.3 FP64 (11.8) and 3.4 us at 40^3
+// (5.3): on small grids the hand-over, some 1.5 us per
 // half-sweep from a store to its sight by the neighbour, is all that is left; at 128^3
-// the shared-memory pipe takes the larger part (24 words per 64 cells and pass).
+// 56% of the issue slots (FP32; FP64, whose d and rd come from L2, 40%) and 44% of the
+// shared-memory pipe are used, and 16 warps wait in turn for shared loads, L2 and the hand-over.
 //
 // The stop rule (GS.f90:11,53).  A sweep ends the solve when no cell of either colour
 // changed by more than zeta.  Every CTA adds the verdict of its red half to a
@@ -179,7 +180,7 @@ __device__ __forceinline__ ResIn<Tc> res_load(const ResRow<Tc>& w, int t, int m,
 // (ring: a cell of the ring; 0 where a row is a cell shorter than the ring).
 //
 // Where d has room on the chip and rd has none, rd is formed from the coefficients: 7.7 us a
-// sweep against 8.4 with rd from L2 on 100x150x150 FP32, 12.6 against 13.6 on 33x150x220
+// sweep against 8.4 with rd from L2 on 100x150x150 FP32, 8.2 against 9.8 on 112^3
 // FP64.  Where d comes from L2 as well, rd does too (formed: 64x128x256 FP64 13.0 us
 // against 12.4).
 template <class Tc, bool EDGE, bool FORM, bool FOUR, class B>

@@ -21,8 +21,8 @@
 // and updated like the brick's own.  1/diag is formed from the coefficients.
 // Rows of at most 32 cells per colour, two or more side by side on a warp's lanes.
 //
-// A sweep takes 2.6 us at 40^3 FP64 (3.3 with two hand-overs), 2.6 us at 61x47x53 FP32 (3.5),
-// 2.7 us at 32x96x96 FP32 (3.8), 1.6 us at 12x10x8 FP64 (2.3, in one CTA).  Bound by the
+// A sweep takes 2.6 us at 40^3 FP64 (3.4 with two hand-overs), 2.7 us at 61x47x53 FP32 (3.5),
+// 2.75 us at 32x96x96 FP32 (3.8), 1.65 us at 12x10x8 FP64 (2.3, in one CTA).  Bound by the
 // hand-over's trip (1.5 us) and, past some 40 rows a brick, by instruction issue: a turn of the 16
 // warps over a row each takes 0.28 us FP32, 0.35 us FP64.  One row per warp and turn: with two, as
 // the resident kernel takes them, half of a small brick's last turn is empty (32x96x96: 2.95 us).

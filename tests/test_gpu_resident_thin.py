@@ -3,8 +3,8 @@ then goes to up to four neighbours) or just fit it in bricks of two, on the
 resident SOR kernel against the streaming path.
 
 Both evaluate the same sweeps in one order of operations, so the sweep counts
-are equal; 1/diag may differ by an ulp in FP64, hence the repository's 1e-12
-for two paths (40 ulp), and 40 ulp of 1 in a last change of 1e-5 or more: 1e-9.
+are equal; the fields are held to the repository's 1e-12 for two paths (40 sweeps of
+at most an ulp), the last change to 40 ulp of 1 in 1e-5 or more: 1e-9.
 """
 import numpy as np
 import pytest
